@@ -1,10 +1,12 @@
 """In-tree build of the native libraries.
 
-Two shared objects are produced under ``eridiffusion_b200/lib``:
+Three shared objects are produced under ``eridiffusion_b200/lib``:
 
 * ``liberi_b200_kernels.so`` — every ``.cu`` file of this directory, compiled for sm_100a only
   (``-gencode arch=compute_100a,code=sm_100a``), exporting plain C entry points that take raw
   device pointers and a stream. Python binds them with ``ctypes`` (see ``ops/_native.py``).
+* ``liberi_b200_torch.so`` — the native op layer (``torch/*.cpp``): the autograd nodes of the public
+  ops, a Python extension module compiled against the installed PyTorch.
 * ``liberi_b200_host.so`` — the C++ host runtime (safetensors mmap reader / writer, pinned staging
   pool, manifest loader worker), no CUDA device code.
 
@@ -121,12 +123,50 @@ def build_host(verbose: bool = False) -> Path:
     return out
 
 
+def build_torch(verbose: bool = False) -> Path:
+    """The op layer of ``torch/*.cpp`` as an extension module (one ``g++ -c`` per file, in parallel)."""
+    import sysconfig
+
+    import torch
+    LIB_DIR.mkdir(exist_ok=True)
+    OBJ_DIR.mkdir(exist_ok=True)
+    root = Path(torch.__file__).resolve().parent
+    cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    out = LIB_DIR / "liberi_b200_torch.so"
+    flags = ["-O2", "-std=c++17", "-fPIC", "-DTORCH_EXTENSION_NAME=liberi_b200_torch", "-DTORCH_API_INCLUDE_EXTENSION_H",
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-isystem", str(root / "include"),
+             "-isystem", str(root / "include/torch/csrc/api/include"), "-isystem", f"{cuda_home}/include",
+             "-isystem", sysconfig.get_paths()["include"]]
+    headers = b"".join(h.read_bytes() for h in (CSRC / "torch" / "eri_ops.h", CSRC / "gemm_args.h"))
+
+    def compile_one(src: Path):
+        obj, stamp = OBJ_DIR / f"torch_{src.stem}.o", OBJ_DIR / f"torch_{src.stem}.sha"
+        dig = hashlib.sha256(src.read_bytes() + headers + " ".join(flags).encode() + torch.__version__.encode()).hexdigest()
+        if obj.exists() and stamp.exists() and stamp.read_text() == dig:
+            return obj, False
+        r = subprocess.run(["g++", *flags, "-c", str(src), "-o", str(obj)], capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"g++ failed for {src.name}:\n{r.stdout}\n{r.stderr}")
+        stamp.write_text(dig)
+        return obj, True
+
+    with cf.ThreadPoolExecutor(max_workers=4) as ex:
+        objs = list(ex.map(compile_one, sorted((CSRC / "torch").glob("*.cpp"))))
+    if any(ch for _, ch in objs) or not out.exists():
+        cmd = ["g++", "-shared", "-o", str(out), *(str(o) for o, _ in objs), f"-L{root / 'lib'}",
+               "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", "-ldl"]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    return out
+
+
 def build_all(verbose: bool = False, ptxas_v: bool = False, debug_bounds: bool | None = None) -> list[Path]:
-    """Kernel library, host library and — with ``debug_bounds`` (default: ``ERI_B200_DEBUG_BOUNDS=1``
+    """Kernel library, host library, op layer and — with ``debug_bounds`` (default: ``ERI_B200_DEBUG_BOUNDS=1``
     in the environment) — the bounds-checked debug variant of the kernel library."""
     if debug_bounds is None:
         debug_bounds = os.environ.get("ERI_B200_DEBUG_BOUNDS") == "1"
-    out = [build_kernels(verbose, ptxas_v), build_host(verbose)]
+    out = [build_kernels(verbose, ptxas_v), build_host(verbose), build_torch(verbose)]
     if debug_bounds:
         out.append(build_kernels(verbose, False, debug_bounds=True))
     return out

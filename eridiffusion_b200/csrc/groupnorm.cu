@@ -1,16 +1,20 @@
 // GroupNorm (+ optional SiLU) for channels-last activations [N, HW, C], forward and backward.
 //
-// Both directions are two bandwidth-bound passes over the activation:
-//   column pass   per-(n, c) sums over HW, accumulated per thread in registers for a fixed group of
-//                 eight channels, combined through shared-memory atomics and one global atomic per
-//                 (n, c, statistic) per CTA:   forward  (sum x, sum x^2)
-//                                              backward (sum dz, sum dz * xhat),  dz = dy * act'(z)
-//   apply pass    forward  y  = act(xhat * w + b)
-//                 backward dx = rstd * (dz * w - s1 / m - xhat * s2 / m)
-// The few-kilobyte reductions between the passes (channels -> groups, parameter gradients) are done
-// by the caller on the [N, C] statistics. The reference's GroupNorm is a forward-only NCHW kernel
-// with one warp-shuffle reduction per group (crates/core/src/cuda/kernels/group_norm.cu); its SDXL
-// ResBlocks apply SiLU as a separate pass (crates/training/src/sdxl/runtime.rs).
+// Each direction is two bandwidth-bound passes over the activation and nothing else:
+//   column pass   per-channel sums over a chunk of rows, one partial record per (n, chunk):
+//                 forward  (sum x, sum x^2) per group;  backward  (sum dz, sum dz * xhat) per channel and,
+//                 weighted by w, per group;  dz = dy * act'(z)
+//   apply pass    first adds the partial records of its sample (in chunk order: results do not depend on timing),
+//                 then forward  y = act(x * a + c) with a = w * rstd, c = b - mean * a held in registers,
+//                 backward dx = rstd * (dz * w - s1 - xhat * s2); the backward's last CTAs add the per-channel
+//                 records into the parameter gradients instead.
+// A thread owns eight fixed channels and walks over rows, so the per-channel constants are loaded once and every
+// access is one 16-byte vector. What bounds it: DRAM (or L2) traffic of the activation, 2 reads + 1 write. The
+// version before used float atomics for the sums and eleven elementwise launches on the [N, C] statistics
+// between the passes: a 1280-channel 32 x 32 layer took 43 us forward, of which 9 us were the two passes.
+// The reference's GroupNorm is a forward-only NCHW kernel with one warp-shuffle reduction per group
+// (crates/core/src/cuda/kernels/group_norm.cu); its SDXL ResBlocks apply SiLU as a separate pass
+// (crates/training/src/sdxl/runtime.rs).
 #include "ptx.cuh"
 
 using namespace eri;
@@ -20,92 +24,203 @@ namespace {
 
 struct GnArgs {
   const bf16 *x, *dy, *w, *b;
-  const float *mean, *rstd;  // [N, G]
-  const float *s1, *s2;      // [N, G] backward group sums (already divided by m)
-  float* stats;              // [N, C, 2]
-  bf16* out;
-  int HW, C, G, silu;
+  float *mean, *rstd;        // [N, G]
+  float* part;               // [N, chunks, G, 2] group records
+  float* part_c;             // [N, chunks, C, 2] channel records (backward)
+  bf16 *out, *dw, *db;
+  int N, HW, C, G, silu, chunks, rows_per_chunk, accumulate, apply_ctas;
+  int gchunks;               // group records per sample that the apply pass adds (1 after a fold)
+  float eps;
 };
 
-__device__ __forceinline__ float act_grad(float z, int silu) {
-  if (!silu) return 1.f;
+constexpr int kUnroll = 4, kMaxThreads = 640;    // up to 5120 channels
+// Partial records an apply CTA adds itself; more are folded by a launch of their own, because every apply CTA
+// re-reads all of them (64 records of 32 groups: 16 KB from L2, about a microsecond).
+constexpr int kMaxDirectChunks = 64;
+
+__device__ __forceinline__ float silu_of(float z) { return z / (1.f + __expf(-z)); }
+__device__ __forceinline__ float silu_grad_of(float z) {
   const float s = 1.f / (1.f + __expf(-z));
   return s * (1.f + z * (1.f - s));
 }
 
-template <int MODE>
-__global__ void gn_colreduce_kernel(const GnArgs a, int rows_per_cta) {
-  extern __shared__ float sacc[];  // [C][2]
-  const int n = blockIdx.y;
-  const int nvec = a.C >> 3;
-  const int R = blockDim.x / nvec;  // rows handled in parallel by the CTA
-  const int v = threadIdx.x % nvec, rr = threadIdx.x / nvec;
-  for (int i = threadIdx.x; i < 2 * a.C; i += blockDim.x) sacc[i] = 0.f;
-  __syncthreads();
-  const int r0 = blockIdx.x * rows_per_cta;
-  const int r1 = min(a.HW, r0 + rows_per_cta);
-  float acc0[8], acc1[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) acc0[j] = acc1[j] = 0.f;
-  float wv[8], bv[8], mu[8], rs[8];
-  if (MODE == 1) {
-    const int cpg = a.C / a.G;
-    float t[8];
-    unpack8(reinterpret_cast<const bf16x8*>(a.w)[v], wv);
-    if (a.b) unpack8(reinterpret_cast<const bf16x8*>(a.b)[v], t);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      bv[j] = a.b ? t[j] : 0.f;
-      const int g = (v * 8 + j) / cpg;
-      mu[j] = a.mean[n * a.G + g];
-      rs[j] = a.rstd[n * a.G + g];
-    }
-  }
-  if (rr < R) {
-    for (int r = r0 + rr; r < r1; r += R) {
-      const size_t off = ((size_t)n * a.HW + r) * a.C;
-      float xv[8];
-      unpack8(reinterpret_cast<const bf16x8*>(a.x + off)[v], xv);
-      if (MODE == 0) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          acc0[j] += xv[j];
-          acc1[j] = fmaf(xv[j], xv[j], acc1[j]);
-        }
-      } else {
-        float g[8];
-        unpack8(reinterpret_cast<const bf16x8*>(a.dy + off)[v], g);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float xh = (xv[j] - mu[j]) * rs[j];
-          const float dz = g[j] * act_grad(fmaf(xh, wv[j], bv[j]), a.silu);
-          acc0[j] += dz;
-          acc1[j] = fmaf(dz, xh, acc1[j]);
-        }
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      atomicAdd(&sacc[(v * 8 + j) * 2], acc0[j]);
-      atomicAdd(&sacc[(v * 8 + j) * 2 + 1], acc1[j]);
-    }
+// Adds the group records of sample n in chunk order into smem s[2 * G].
+__device__ __forceinline__ void fold_groups(const GnArgs& a, int n, float* s) {
+  const float* p = a.part + (size_t)n * a.gchunks * a.G * 2;
+  for (int i = threadIdx.x; i < 2 * a.G; i += blockDim.x) {
+    float v = 0.f;
+#pragma unroll 8
+    for (int c = 0; c < a.gchunks; ++c) v += p[(size_t)c * a.G * 2 + i];
+    s[i] = v;
   }
   __syncthreads();
-  float* dst = a.stats + (size_t)n * a.C * 2;
-  for (int i = threadIdx.x; i < 2 * a.C; i += blockDim.x) atomicAdd(&dst[i], sacc[i]);
 }
 
-template <int MODE>
-__global__ void gn_apply_kernel(const GnArgs a, long long total_vec) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= total_vec) return;
-  const int nvec = a.C >> 3;
-  const int v = (int)(i % nvec);
-  const long long row = i / nvec;
-  const int n = (int)(row / a.HW);
+template <bool BWD>
+__global__ void __launch_bounds__(kMaxThreads) gn_column_kernel(const GnArgs a) {
+  extern __shared__ float sm[];     // [R][C][2] partial sums of the CTA's row lanes
+  const int n = blockIdx.y, nvec = a.C >> 3;
+  const int R = blockDim.x / nvec;
+  const int v = threadIdx.x % nvec, rr = threadIdx.x / nvec;
+  const int r0 = blockIdx.x * a.rows_per_chunk, r1 = min(a.HW, r0 + a.rows_per_chunk);
+  float s0[8], s1[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) s0[j] = s1[j] = 0.f;
+  const bf16x8* xp = reinterpret_cast<const bf16x8*>(a.x + (size_t)n * a.HW * a.C) + v;
+  if (rr < R) {
+    if constexpr (!BWD) {
+      for (int r = r0 + rr; r < r1; r += R * kUnroll) {
+        bf16x8 q[kUnroll];
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u)
+          if (r + u * R < r1) q[u] = xp[(size_t)(r + u * R) * nvec];
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u)
+          if (r + u * R < r1) {
+            float f[8];
+            unpack8(q[u], f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              s0[j] += f[j];
+              s1[j] = fmaf(f[j], f[j], s1[j]);
+            }
+          }
+      }
+    } else {
+      const bf16x8* gp = reinterpret_cast<const bf16x8*>(a.dy + (size_t)n * a.HW * a.C) + v;
+      const int cpg = a.C / a.G;
+      float wv[8], bv[8], mu[8], rs[8];
+      unpack8(reinterpret_cast<const bf16x8*>(a.w)[v], wv);
+      if (a.b) {
+        unpack8(reinterpret_cast<const bf16x8*>(a.b)[v], bv);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) bv[j] = 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int g = (v * 8 + j) / cpg;
+        mu[j] = a.mean[n * a.G + g];
+        rs[j] = a.rstd[n * a.G + g];
+      }
+      for (int r = r0 + rr; r < r1; r += R * 2) {
+        bf16x8 q[2], d[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          if (r + u * R < r1) {
+            q[u] = xp[(size_t)(r + u * R) * nvec];
+            d[u] = gp[(size_t)(r + u * R) * nvec];
+          }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          if (r + u * R < r1) {
+            float f[8], g[8];
+            unpack8(q[u], f);
+            unpack8(d[u], g);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const float xh = (f[j] - mu[j]) * rs[j];
+              const float dz = a.silu ? g[j] * silu_grad_of(fmaf(xh, wv[j], bv[j])) : g[j];
+              s0[j] += dz;
+              s1[j] = fmaf(dz, xh, s1[j]);
+            }
+          }
+      }
+    }
+    float* o = sm + ((size_t)rr * a.C + v * 8) * 2;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      o[2 * j] = s0[j];
+      o[2 * j + 1] = s1[j];
+    }
+  }
+  __syncthreads();
+  // row lanes -> one record per channel, in the first lane's slots
+  for (int i = threadIdx.x; i < 2 * a.C; i += blockDim.x) {
+    float t = sm[i];
+    for (int r = 1; r < R; ++r) t += sm[(size_t)r * a.C * 2 + i];
+    if constexpr (BWD) {
+      a.part_c[((size_t)n * a.chunks + blockIdx.x) * a.C * 2 + i] = t;
+      t *= __bfloat162float(a.w[i >> 1]);
+    }
+    sm[i] = t;
+  }
+  __syncthreads();
   const int cpg = a.C / a.G;
-  float xv[8], wv[8], bv[8], o[8];
-  unpack8(reinterpret_cast<const bf16x8*>(a.x)[i], xv);
+  float* dst = a.part + ((size_t)n * a.chunks + blockIdx.x) * a.G * 2;
+  for (int i = threadIdx.x; i < 2 * a.G; i += blockDim.x) {
+    const int g = i >> 1;
+    float t = 0.f;
+    for (int c = 0; c < cpg; ++c) t += sm[(g * cpg + c) * 2 + (i & 1)];
+    dst[i] = t;
+  }
+}
+
+// Many chunks: their group records folded into one (one CTA per sample).
+__global__ void gn_fold_kernel(GnArgs a, float* folded) {
+  const int n = blockIdx.x, lanes = blockDim.x / (2 * a.G);
+  extern __shared__ float sm[];     // [lanes][2 * G]
+  const int i = threadIdx.x % (2 * a.G), l = threadIdx.x / (2 * a.G);
+  const float* p = a.part + (size_t)n * a.chunks * a.G * 2;
+  if (l < lanes) {
+    float v = 0.f;
+#pragma unroll 8
+    for (int c = l; c < a.chunks; c += lanes) v += p[(size_t)c * a.G * 2 + i];
+    sm[l * 2 * a.G + i] = v;
+  }
+  __syncthreads();
+  if (l == 0) {
+    float v = 0.f;
+    for (int k = 0; k < lanes; ++k) v += sm[k * 2 * a.G + i];
+    folded[(size_t)n * a.G * 2 + i] = v;
+  }
+}
+
+template <bool BWD>
+__global__ void __launch_bounds__(kMaxThreads) gn_apply_kernel(const GnArgs a) {
+  extern __shared__ float sm[];     // [2 * G]
+  const int nvec = a.C >> 3;
+  if (BWD && (int)blockIdx.x >= a.apply_ctas) {
+    // parameter gradients: one warp-row of lanes per eight channels would be idle work for the apply CTAs
+    if (blockIdx.y) return;
+    const int cta = blockIdx.x - a.apply_ctas, per = blockDim.x / 8;     // eight record lanes per channel pair slot
+    const int i = cta * per + (int)threadIdx.x / 8, l = threadIdx.x & 7;   // i: index into [C][2]
+    float t = 0.f;
+    if (i < 2 * a.C) {
+      const int total = a.N * a.chunks;
+      for (int c = l; c < total; c += 8) t += a.part_c[(size_t)c * a.C * 2 + i];
+    }
+#pragma unroll
+    for (int o = 4; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (i < 2 * a.C && l == 0) {
+      bf16* dst = (i & 1) ? a.dw : a.db;
+      if (dst) {
+        if (a.accumulate & ((i & 1) ? 1 : 2)) t += __bfloat162float(dst[i >> 1]);
+        dst[i >> 1] = __float2bfloat16(t);
+      }
+    }
+    return;
+  }
+  const int n = blockIdx.y, cpg = a.C / a.G;
+  const float inv_m = 1.f / ((float)a.HW * (float)cpg);
+  fold_groups(a, n, sm);
+  if constexpr (!BWD) {
+    for (int g = threadIdx.x; g < a.G; g += blockDim.x) {
+      const float mean = sm[2 * g] * inv_m;
+      const float rstd = rsqrtf(fmaxf(sm[2 * g + 1] * inv_m - mean * mean, 0.f) + a.eps);
+      sm[2 * g] = mean;
+      sm[2 * g + 1] = rstd;
+      if (blockIdx.x == 0 && a.mean) {
+        a.mean[n * a.G + g] = mean;
+        a.rstd[n * a.G + g] = rstd;
+      }
+    }
+    __syncthreads();
+  }
+  const int R = blockDim.x / nvec;
+  const int v = threadIdx.x % nvec, rr = threadIdx.x / nvec;
+  if (rr >= R) return;
+  float wv[8], bv[8];
   unpack8(reinterpret_cast<const bf16x8*>(a.w)[v], wv);
   if (a.b) {
     unpack8(reinterpret_cast<const bf16x8*>(a.b)[v], bv);
@@ -113,42 +228,123 @@ __global__ void gn_apply_kernel(const GnArgs a, long long total_vec) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) bv[j] = 0.f;
   }
-  if (MODE == 0) {
+  const size_t base = (size_t)n * a.HW * nvec + v;
+  const bf16x8* xp = reinterpret_cast<const bf16x8*>(a.x) + base;
+  bf16x8* op = reinterpret_cast<bf16x8*>(a.out) + base;
+  const int step = a.apply_ctas * R;
+  if constexpr (!BWD) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int g = (v * 8 + j) / cpg;
-      const float xh = (xv[j] - a.mean[n * a.G + g]) * a.rstd[n * a.G + g];
-      const float z = fmaf(xh, wv[j], bv[j]);
-      o[j] = a.silu ? z / (1.f + __expf(-z)) : z;
+      wv[j] *= sm[2 * g + 1];
+      bv[j] = fmaf(-sm[2 * g], wv[j], bv[j]);
+    }
+    for (int r = blockIdx.x * R + rr; r < a.HW; r += step * kUnroll) {
+      bf16x8 q[kUnroll];
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u)
+        if (r + u * step < a.HW) q[u] = xp[(size_t)(r + u * step) * nvec];
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u)
+        if (r + u * step < a.HW) {
+          float f[8];
+          unpack8(q[u], f);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float z = fmaf(f[j], wv[j], bv[j]);
+            f[j] = a.silu ? silu_of(z) : z;
+          }
+          op[(size_t)(r + u * step) * nvec] = pack8(f);
+        }
     }
   } else {
-    float g8[8];
-    unpack8(reinterpret_cast<const bf16x8*>(a.dy)[i], g8);
+    const bf16x8* gp = reinterpret_cast<const bf16x8*>(a.dy) + base;
+    float mu[8], rs[8], t1[8], t2[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int g = (v * 8 + j) / cpg;
-      const float rs = a.rstd[n * a.G + g];
-      const float xh = (xv[j] - a.mean[n * a.G + g]) * rs;
-      const float dz = g8[j] * act_grad(fmaf(xh, wv[j], bv[j]), a.silu);
-      o[j] = rs * (dz * wv[j] - a.s1[n * a.G + g] - xh * a.s2[n * a.G + g]);
+      mu[j] = a.mean[n * a.G + g];
+      rs[j] = a.rstd[n * a.G + g];
+      t1[j] = sm[2 * g] * inv_m;
+      t2[j] = sm[2 * g + 1] * inv_m;
+    }
+    for (int r = blockIdx.x * R + rr; r < a.HW; r += step * 2) {
+      bf16x8 q[2], d[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        if (r + u * step < a.HW) {
+          q[u] = xp[(size_t)(r + u * step) * nvec];
+          d[u] = gp[(size_t)(r + u * step) * nvec];
+        }
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        if (r + u * step < a.HW) {
+          float f[8], g[8];
+          unpack8(q[u], f);
+          unpack8(d[u], g);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float xh = (f[j] - mu[j]) * rs[j];
+            const float dz = a.silu ? g[j] * silu_grad_of(fmaf(xh, wv[j], bv[j])) : g[j];
+            f[j] = rs[j] * (dz * wv[j] - t1[j] - xh * t2[j]);
+          }
+          op[(size_t)(r + u * step) * nvec] = pack8(f);
+        }
     }
   }
-  reinterpret_cast<bf16x8*>(a.out)[i] = pack8(o);
 }
 
-template <int MODE>
-int launch_colreduce(const GnArgs& a, int N, cudaStream_t st) {
-  const int nvec = a.C >> 3;
-  if (nvec > 1024) return -1;
-  int R = 256 / nvec;
-  if (R < 1) R = 1;
-  const int threads = ((R * nvec + 31) / 32) * 32;
-  // enough CTAs to fill the machine a few times over, at least 32 rows each
-  int rows_per_cta = (int)(((long long)a.HW * N + 148 * 8 - 1) / (148 * 8));
-  if (rows_per_cta < 32) rows_per_cta = 32;
-  rows_per_cta = (rows_per_cta + R - 1) / R * R;
-  dim3 grid((a.HW + rows_per_cta - 1) / rows_per_cta, N);
-  gn_colreduce_kernel<MODE><<<grid, threads, 2 * a.C * sizeof(float), st>>>(a, rows_per_cta);
+struct GnPlan {
+  int threads, R, chunks, rows_per_chunk, apply_ctas;
+};
+
+// At least four rows per thread and about four column CTAs per SM; the apply pass about eight per SM.
+GnPlan plan_for(int N, int HW, int C) {
+  GnPlan p;
+  const int nvec = C >> 3;
+  p.R = 256 / nvec;
+  if (p.R < 1) p.R = 1;
+  p.threads = (p.R * nvec + 31) / 32 * 32;
+  const int min_rows = p.R * kUnroll;
+  int want = (148 * 4 + N - 1) / N;
+  int rows = (HW + want - 1) / want;
+  rows = (rows + min_rows - 1) / min_rows * min_rows;
+  p.rows_per_chunk = rows;
+  p.chunks = (HW + rows - 1) / rows;
+  int ctas = (148 * 8 + N - 1) / N;
+  const int most = (HW + p.R * 2 - 1) / (p.R * 2);
+  p.apply_ctas = ctas < most ? ctas : most;
+  return p;
+}
+
+template <bool BWD>
+int run(GnArgs a, float* ws, cudaStream_t st) {
+  const GnPlan p = plan_for(a.N, a.HW, a.C);
+  if (p.threads > kMaxThreads || 2 * a.G > 1024) return -1;
+  a.chunks = a.gchunks = p.chunks;
+  a.rows_per_chunk = p.rows_per_chunk;
+  a.apply_ctas = p.apply_ctas;
+  a.part = ws;
+  float* folded = ws + (size_t)a.N * p.chunks * a.G * 2;
+  a.part_c = folded + (size_t)a.N * a.G * 2;
+  const int smem = p.R * a.C * 2 * (int)sizeof(float);
+  static bool configured[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -2;
+  if (!configured[dev]) {
+    if (cudaFuncSetAttribute(gn_column_kernel<BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536) != cudaSuccess)
+      return -2;
+    configured[dev] = true;
+  }
+  gn_column_kernel<BWD><<<dim3(p.chunks, a.N), p.threads, smem, st>>>(a);
+  if (p.chunks > kMaxDirectChunks) {
+    const int lanes = 1024 / (2 * a.G) < 1 ? 1 : 1024 / (2 * a.G);
+    gn_fold_kernel<<<a.N, lanes * 2 * a.G, lanes * 2 * a.G * sizeof(float), st>>>(a, folded);
+    a.part = folded;
+    a.gchunks = 1;
+  }
+  const int extra = BWD && (a.dw || a.db) ? (2 * a.C + p.threads / 8 - 1) / (p.threads / 8) : 0;
+  gn_apply_kernel<BWD><<<dim3(p.apply_ctas + extra, a.N), p.threads, 2 * a.G * sizeof(float), st>>>(a);
   return (int)cudaGetLastError();
 }
 
@@ -156,48 +352,32 @@ int launch_colreduce(const GnArgs& a, int N, cudaStream_t st) {
 
 extern "C" {
 
-// stats [N, C, 2] fp32 must be zero on entry. Forward: (sum x, sum x^2) per (n, c).
-int eri_gn_stats_fwd(const void* x, float* stats, int N, int HW, int C, void* stream) {
-  if (C % 8) return -1;
-  GnArgs a = {};
-  a.x = (const bf16*)x; a.stats = stats; a.HW = HW; a.C = C; a.G = 1;
-  return launch_colreduce<0>(a, N, (cudaStream_t)stream);
+// fp32 words of workspace one call needs.
+long long eri_gn_workspace(int N, int HW, int C, int G, int backward) {
+  const GnPlan p = plan_for(N, HW, C);
+  return (long long)N * (p.chunks + 1) * G * 2 + (backward ? (long long)N * p.chunks * C * 2 : 0);
 }
 
-int eri_gn_apply_fwd(const void* x, const void* w, const void* b, const float* mean, const float* rstd,
-                     void* y, int N, int HW, int C, int G, int silu, void* stream) {
+// y = act(GroupNorm(x)); mean / rstd [N, G] are written for the backward when given.
+int eri_gn_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, float* ws, int N, int HW,
+               int C, int G, float eps, int silu, void* stream) {
   if (C % 8 || C % G) return -1;
   GnArgs a = {};
-  a.x = (const bf16*)x; a.w = (const bf16*)w; a.b = (const bf16*)b; a.mean = mean; a.rstd = rstd;
-  a.out = (bf16*)y; a.HW = HW; a.C = C; a.G = G; a.silu = silu;
-  const long long total = (long long)N * HW * (C >> 3);
-  gn_apply_kernel<0><<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(a, total);
-  return (int)cudaGetLastError();
+  a.x = (const bf16*)x; a.w = (const bf16*)w; a.b = (const bf16*)b; a.out = (bf16*)y; a.mean = mean; a.rstd = rstd;
+  a.N = N; a.HW = HW; a.C = C; a.G = G; a.silu = silu; a.eps = eps;
+  return run<false>(a, ws, (cudaStream_t)stream);
 }
 
-// Backward column sums: stats[n, c] = (sum dz, sum dz * xhat), zero on entry.
-int eri_gn_stats_bwd(const void* x, const void* dy, const void* w, const void* b, const float* mean,
-                     const float* rstd, float* stats, int N, int HW, int C, int G, int silu,
-                     void* stream) {
+// dx, and the parameter gradients dw / db [C] (bf16; null: not wanted). accumulate: bit 0 adds into dw, bit 1 into db.
+int eri_gn_bwd(const void* x, const void* dy, const void* w, const void* b, const float* mean, const float* rstd, void* dx,
+               void* dw, void* db, float* ws, int N, int HW, int C, int G, int silu, int accumulate, void* stream) {
   if (C % 8 || C % G) return -1;
   GnArgs a = {};
   a.x = (const bf16*)x; a.dy = (const bf16*)dy; a.w = (const bf16*)w; a.b = (const bf16*)b;
-  a.mean = mean; a.rstd = rstd; a.stats = stats; a.HW = HW; a.C = C; a.G = G; a.silu = silu;
-  return launch_colreduce<1>(a, N, (cudaStream_t)stream);
-}
-
-// s1, s2 [N, G]: group sums of w*sum(dz) and w*sum(dz*xhat), each divided by m = HW * C / G.
-int eri_gn_apply_bwd(const void* x, const void* dy, const void* w, const void* b, const float* mean,
-                     const float* rstd, const float* s1, const float* s2, void* dx, int N, int HW,
-                     int C, int G, int silu, void* stream) {
-  if (C % 8 || C % G) return -1;
-  GnArgs a = {};
-  a.x = (const bf16*)x; a.dy = (const bf16*)dy; a.w = (const bf16*)w; a.b = (const bf16*)b;
-  a.mean = mean; a.rstd = rstd; a.s1 = s1; a.s2 = s2; a.out = (bf16*)dx;
-  a.HW = HW; a.C = C; a.G = G; a.silu = silu;
-  const long long total = (long long)N * HW * (C >> 3);
-  gn_apply_kernel<1><<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(a, total);
-  return (int)cudaGetLastError();
+  a.mean = const_cast<float*>(mean); a.rstd = const_cast<float*>(rstd);
+  a.out = (bf16*)dx; a.dw = (bf16*)dw; a.db = (bf16*)db;
+  a.N = N; a.HW = HW; a.C = C; a.G = G; a.silu = silu; a.accumulate = accumulate;
+  return run<true>(a, ws, (cudaStream_t)stream);
 }
 
 }  // extern "C"

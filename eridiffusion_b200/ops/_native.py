@@ -20,6 +20,7 @@ DEBUG_BOUNDS = os.environ.get("ERI_B200_DEBUG_BOUNDS") == "1"
 _LIB_PATH = _PKG / "lib" / ("liberi_b200_kernels_debug.so" if DEBUG_BOUNDS else "liberi_b200_kernels.so")
 _lock = threading.Lock()
 _lib = None
+_ops = None
 _launches = 0  # number of kernel launches issued through this module (for bench accounting)
 
 
@@ -98,10 +99,6 @@ _SIGNATURES = {
     "eri_adamw32_step": [_P, _P, _P, _P, _P, _L, _I, _F, _F, _F, _F, _F, _I, _F, _F, _U32, _I, _P],
     "eri_ema_update": [_P, _P, _L, _F, _P],
     "eri_scale_bf16": [_P, _L, _P, _F, _F, _P],
-    "eri_gn_stats_fwd": [_P, _P, _I, _I, _I, _P],
-    "eri_gn_apply_fwd": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
-    "eri_gn_stats_bwd": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
-    "eri_gn_apply_bwd": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "eri_row_l2norm": [_P, _P, _L, _I, _P],
     "eri_topk_desc": [_P, _P, _I, _I, _I, _P],
     "eri_build_inverse": [_P, _P, _I, _I, _I, _P],
@@ -208,6 +205,32 @@ def require():
     return h
 
 
+def ops():
+    """The native op layer (``csrc/torch``): autograd nodes that launch the kernels without going through
+    Python. Loaded on the first use of a CUDA op; a missing module is an error, never a fallback."""
+    global _ops
+    if _ops is None:
+        require()
+        path = _PKG / "lib" / "liberi_b200_torch.so"
+        with _lock:
+            if _ops is None:
+                try:
+                    if not path.exists() and os.environ.get("ERI_B200_NO_BUILD") != "1":
+                        from ..csrc import build as _b
+                        _b.build_torch()
+                    from importlib.machinery import ExtensionFileLoader
+                    from importlib.util import module_from_spec, spec_from_loader
+                    loader = ExtensionFileLoader("liberi_b200_torch", str(path))
+                    mod = module_from_spec(spec_from_loader("liberi_b200_torch", loader))
+                    loader.exec_module(mod)
+                    mod.init(str(_LIB_PATH))
+                except Exception as e:
+                    raise NativeLibraryError(f"native op layer {path} is missing or failed to load ({e}); run "
+                                             "`python -m eridiffusion_b200.csrc.build`") from e
+                _ops = mod
+    return _ops
+
+
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 _raw_device = getattr(torch._C, "_cuda_getDevice", None)
 
@@ -233,4 +256,4 @@ def check(code: int, what: str) -> None:
 
 
 def launch_count() -> int:
-    return _launches
+    return _launches + (_ops.launch_count() if _ops is not None else 0)

@@ -262,13 +262,12 @@ def check_error() -> int:
     return e
 
 
-class _FlashAttention(torch.autograd.Function):
+class _IntoBuffer(torch.autograd.Function):
+    """Attention written in place into a buffer the caller owns (one that peers read)."""
+
     @staticmethod
-    def forward(ctx, q, k, v, scale, out_buf=None, kbias=None):
-        if out_buf is not None:
-            ctx.mark_dirty(out_buf)          # an input that is written in place and returned
-        if kbias is None and k.shape[1] < 128:
-            kbias = key_bias(None, k.shape[0], k.shape[1], q.device)
+    def forward(ctx, q, k, v, scale, out_buf, kbias):
+        ctx.mark_dirty(out_buf)
         out, lse = fwd(q, k, v, scale, out_buf, kbias)
         ctx.save_for_backward(q, k, v, out, lse, kbias)
         ctx.scale = scale
@@ -277,22 +276,16 @@ class _FlashAttention(torch.autograd.Function):
     @staticmethod
     def backward(ctx, do):
         q, k, v, out, lse, kbias = ctx.saved_tensors
-        do = do.contiguous()
-        if has_backward():
-            dq, dk, dv = bwd(do, q, k, v, out, lse, ctx.scale, kbias)
-            return dq, dk, dv, None, None, None
-        if kbias is not None:
-            raise RuntimeError("masked flash attention needs the native backward kernels")
-        # Library recompute path, used only while the native backward is absent from the build.
-        from . import reference as R
-        with torch.enable_grad():
-            qq, kk, vv = (t.detach().requires_grad_() for t in (q, k, v))
-            o = R.attention(qq, kk, vv, ctx.scale)
-        dq, dk, dv = torch.autograd.grad(o, (qq, kk, vv), do)
-        return dq, dk, dv, None, None, None
+        return (*bwd(do.contiguous(), q, k, v, out, lse, ctx.scale, kbias), None, None, None)
 
 
 def flash_attention(q, k, v, scale=None, out=None, mask=None):
-    """``mask``: None or a key-only mask (see ``mask_is_key_only``); the bias row is built here."""
+    """Differentiable attention on the kernels. ``mask``: None or a key-only mask (see ``mask_is_key_only``);
+    the bias row is built here. ``out``: optional destination, written in place and returned."""
     kbias = None if mask is None else key_bias(mask, q.shape[0], k.shape[1], q.device)
-    return _FlashAttention.apply(q, k, v, scale, out, kbias)
+    if out is not None:
+        if kbias is None and k.shape[1] < 128:
+            kbias = key_bias(None, k.shape[0], k.shape[1], q.device)
+        return _IntoBuffer.apply(q, k, v, scale, out, kbias)
+    poly = _poly_pairs() if _PAIR_ENABLED and pair_forward_ok(q.device) else -1
+    return N.ops().attention(q, k, v, scale if scale is not None else 1.0 / math.sqrt(q.shape[-1]), kbias, poly)

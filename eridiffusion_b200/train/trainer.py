@@ -261,7 +261,7 @@ class Trainer:
                 self.grad_sync.gather_params()
         self.arena.zero_grad()
         if self._lora_mats:
-            F.invalidate_lora_transposes()
+            F.invalidate_lora_transposes(self._lora_mats)
             self._lora_t_stale = True
         if self.ema is not None:
             self.ema.update()
