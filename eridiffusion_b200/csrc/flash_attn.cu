@@ -27,6 +27,7 @@
 
 #include "ptx.cuh"
 #include "tma_host.h"
+#include "attn_args.h"
 
 using namespace eri;
 typedef __nv_bfloat16 bf16;
@@ -421,19 +422,22 @@ int poly_pairs() {
   return v;
 }
 
-int make_qkv_map(CUtensorMap* m, const void* ptr, int B, int L, int H, int DH) {
+int make_qkv_map(CUtensorMap* m, const void* ptr, int B, int L, int H, int DH, long long ld) {
   uint64_t dims[3] = {(uint64_t)H * DH, (uint64_t)L, (uint64_t)B};
-  uint64_t strides[2] = {(uint64_t)H * DH * 2, (uint64_t)L * H * DH * 2};
+  uint64_t strides[2] = {(uint64_t)ld * 2, (uint64_t)L * ld * 2};
   uint32_t box[3] = {64, 128, 1};
   return make_tensor_map(m, ptr, 3, dims, strides, box, 128);
 }
 
 int fwd_entry(const void* q, const void* k, const void* v, void* out, float* lse, const float* kbias,
-              int B, int H, int Lq, int Lk, int DH, float scale, void* stream, long long out_ld = 0) {
+              int B, int H, int Lq, int Lk, int DH, float scale, void* stream, EriAttnStrides ld = {}) {
   if (DH != 64 && DH != 128) return -1;
-  if (out_ld == 0) out_ld = (long long)H * DH;
-  // rows are written as 16-byte words
-  if (out_ld < (long long)H * DH || out_ld % 8 || (((uintptr_t)out) & 15)) return -7;
+  // rows are read by TMA and written as 16-byte words
+  for (long long* t : {&ld.q, &ld.k, &ld.v, &ld.out}) {
+    if (*t == 0) *t = (long long)H * DH;
+    if (*t < (long long)H * DH || *t % 8) return -7;
+  }
+  if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out) & 15) return -7;
   // Fewer than 128 keys (one mostly empty tile) need the key bias to blank the padding; queries are
   // tiled by 128 rows and a short last tile is simply not written back.
   if (Lq < 1 || Lk < 1 || (Lk < 128 && !kbias)) return -2;
@@ -444,13 +448,13 @@ int fwd_entry(const void* q, const void* k, const void* v, void* out, float* lse
     cudaMemset(g_fa_err[dev], 0, sizeof(int));
   }
   CUtensorMap tq, tk, tv;
-  if (make_qkv_map(&tq, q, B, Lq, H, DH) || make_qkv_map(&tk, k, B, Lk, H, DH) ||
-      make_qkv_map(&tv, v, B, Lk, H, DH))
+  if (make_qkv_map(&tq, q, B, Lq, H, DH, ld.q) || make_qkv_map(&tk, k, B, Lk, H, DH, ld.k) ||
+      make_qkv_map(&tv, v, B, Lk, H, DH, ld.v))
     return -4;
   FaParams p;
   p.B = B; p.H = H; p.Lq = Lq; p.Lk = Lk;
   p.scale_log2 = scale * 1.4426950408889634f;
-  p.out = (bf16*)out; p.out_ld = out_ld; p.lse = lse; p.err = g_fa_err[dev];
+  p.out = (bf16*)out; p.out_ld = ld.out; p.lse = lse; p.err = g_fa_err[dev];
   p.kbias = kbias; p.Lkb = (Lk + BKV - 1) / BKV * BKV;
   cudaStream_t st = (cudaStream_t)stream;
   if (kbias) {
@@ -495,7 +499,15 @@ int eri_flash_attn_fwd(const void* q, const void* k, const void* v, void* out, f
 // of a wider matrix (the attention half of a single-stream block's second linear's input) in place.
 int eri_flash_attn_fwd_ld(const void* q, const void* k, const void* v, void* out, float* lse, int B,
                           int H, int Lq, int Lk, int DH, float scale, long long out_ld, void* stream) {
-  return fwd_entry(q, k, v, out, lse, nullptr, B, H, Lq, Lk, DH, scale, stream, out_ld);
+  EriAttnStrides ld = {};
+  ld.out = out_ld;
+  return fwd_entry(q, k, v, out, lse, nullptr, B, H, Lq, Lk, DH, scale, stream, ld);
+}
+
+// Any of the operands a column block of a wider matrix (attn_args.h); kbias may be null when Lk >= 128.
+int eri_flash_attn_fwd_strided(const void* q, const void* k, const void* v, void* out, float* lse, const float* kbias, int B,
+                               int H, int Lq, int Lk, int DH, float scale, const EriAttnStrides* ld, void* stream) {
+  return fwd_entry(q, k, v, out, lse, kbias, B, H, Lq, Lk, DH, scale, stream, *ld);
 }
 
 // The same with an additive key bias: kbias [B, ceil(Lk/128)*128] fp32 in log2 units (the caller

@@ -18,6 +18,7 @@
 
 #include "ptx.cuh"
 #include "tma_host.h"
+#include "attn_args.h"
 
 using namespace eri;
 typedef __nv_bfloat16 bf16;
@@ -40,6 +41,7 @@ struct FaBwdParams {
   const float* kbias;    // MASK variants: [B, Lkb] additive key bias in log2 units (-1e30 = masked),
                          // followed by one int per (batch, 128-key tile): 1 = the tile has a non-zero bias
   int Lkb;               // ceil(Lk / 128) * 128
+  long long q_ld, dq_ld, dk_ld, dv_ld;   // token strides, H * DH when contiguous
 };
 
 constexpr int T = 128;  // tile edge (queries and keys)
@@ -371,7 +373,8 @@ fa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     if (ok) {
       tc_fence_after();
       const int kv = k0 + qd * 32 + lane;
-      const size_t obase = (((size_t)b * p.Lk + kv) * p.H + h) * DH;
+      bf16* dv_row = p.dv + ((size_t)b * p.Lk + kv) * p.dv_ld + (size_t)h * DH;
+      bf16* dk_row = p.dk + ((size_t)b * p.Lk + kv) * p.dk_ld + (size_t)h * DH;
 #pragma unroll 1
       for (int c = sub; c < DH / 32; c += 4) {
         uint32_t rv[32], rk[32];
@@ -387,8 +390,8 @@ fa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
               a[x] = __uint_as_float(rv[g * 8 + x]);
               bb[x] = __uint_as_float(rk[g * 8 + x]) * p.scale;
             }
-            *reinterpret_cast<bf16x8*>(p.dv + obase + c * 32 + g * 8) = pack8(a);
-            *reinterpret_cast<bf16x8*>(p.dk + obase + c * 32 + g * 8) = pack8(bb);
+            *reinterpret_cast<bf16x8*>(dv_row + c * 32 + g * 8) = pack8(a);
+            *reinterpret_cast<bf16x8*>(dk_row + c * 32 + g * 8) = pack8(bb);
           }
         }
       }
@@ -595,7 +598,7 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     {
       // Stage Q as a constant A operand: warp groups 0 and 1 copy one half of the row block
       // each, every thread its own query row (= TMEM lane), straight from global memory.
-      const bf16* src = p.q + (((size_t)b * p.Lq + row) * p.H + h) * DH + (sub & 1) * (DH / 2);
+      const bf16* src = p.q + ((size_t)b * p.Lq + row) * p.q_ld + (size_t)h * DH + (sub & 1) * (DH / 2);
       const uint32_t dst = lane_addr + QA_COL + (sub & 1) * (DH / 4);
 #pragma unroll
       for (int w = 0; w < (sub < 2 ? DH / 64 : 0); ++w) {
@@ -720,7 +723,7 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
     if (ok) {
       tc_fence_after();
-      const size_t obase = (((size_t)b * p.Lq + row) * p.H + h) * DH;
+      bf16* dq_row = p.dq + ((size_t)b * p.Lq + row) * p.dq_ld + (size_t)h * DH;
 #pragma unroll 1
       for (int c = sub; c < DH / 32; c += 4) {
         uint32_t r[32];
@@ -732,7 +735,7 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             float a[8];
 #pragma unroll
             for (int x = 0; x < 8; ++x) a[x] = __uint_as_float(r[g * 8 + x]) * p.scale;
-            *reinterpret_cast<bf16x8*>(p.dq + obase + c * 32 + g * 8) = pack8(a);
+            *reinterpret_cast<bf16x8*>(dq_row + c * 32 + g * 8) = pack8(a);
           }
         }
       }
@@ -752,9 +755,9 @@ long long* g_fab_trace = nullptr;
 int g_fab_trace_cap = 0;
 int g_fab_trace_kernel = 0;  // 0: dQ kernel, 1: dK/dV kernel
 
-int make_map(CUtensorMap* m, const void* ptr, int B, int L, int H, int DH) {
+int make_map(CUtensorMap* m, const void* ptr, int B, int L, int H, int DH, long long ld) {
   uint64_t dims[3] = {(uint64_t)H * DH, (uint64_t)L, (uint64_t)B};
-  uint64_t strides[2] = {(uint64_t)H * DH * 2, (uint64_t)L * H * DH * 2};
+  uint64_t strides[2] = {(uint64_t)ld * 2, (uint64_t)L * ld * 2};
   uint32_t box[3] = {64, 128, 1};
   return make_tensor_map(m, ptr, 3, dims, strides, box, 128);
 }
@@ -821,11 +824,17 @@ void launch_prep(const void* out, const void* dout, const float* lse, float* lse
 int bwd_entry(const void* dout, const void* q, const void* k, const void* v, const void* out,
               const float* lse, float* lse2, float* delta, void* dq, void* dk, void* dv,
               const float* kbias, int B, int H, int Lq, int Lk, int DH, float scale, void* stream,
-              long long out_ld = 0) {
+              EriAttnStrides ld = {}) {
   if (DH != 64 && DH != 128) return -1;
   if (Lq < 1 || Lk < 1 || (Lk < 128 && !kbias)) return -2;
   if (kbias && (((uintptr_t)kbias) & 15)) return -6;
-  if (out_ld && (out_ld < (long long)H * DH || out_ld % 8 || (((uintptr_t)out) & 15))) return -7;
+  for (long long* t : {&ld.q, &ld.k, &ld.v, &ld.out, &ld.dq, &ld.dk, &ld.dv}) {
+    if (*t == 0) *t = (long long)H * DH;
+    if (*t < (long long)H * DH || *t % 8) return -7;
+  }
+  if (((uintptr_t)dout | (uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out | (uintptr_t)dq | (uintptr_t)dk |
+       (uintptr_t)dv) & 15)
+    return -7;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -3;
   if (!g_fab_err[dev]) {
@@ -835,10 +844,10 @@ int bwd_entry(const void* dout, const void* q, const void* k, const void* v, con
   cudaStream_t st = (cudaStream_t)stream;
   const int Lp = (Lq + T - 1) / T * T;
   CUtensorMap tq, tk, tv, td;
-  if (make_map(&tq, q, B, Lq, H, DH) || make_map(&tk, k, B, Lk, H, DH) ||
-      make_map(&tv, v, B, Lk, H, DH) || make_map(&td, dout, B, Lq, H, DH))
+  if (make_map(&tq, q, B, Lq, H, DH, ld.q) || make_map(&tk, k, B, Lk, H, DH, ld.k) ||
+      make_map(&tv, v, B, Lk, H, DH, ld.v) || make_map(&td, dout, B, Lq, H, DH, (long long)H * DH))
     return -4;
-  launch_prep(out, dout, lse, lse2, delta, B, H, Lq, Lp, DH, st, out_ld);
+  launch_prep(out, dout, lse, lse2, delta, B, H, Lq, Lp, DH, st, ld.out);
   FaBwdParams p;
   p.B = B; p.H = H; p.Lq = Lq; p.Lk = Lk; p.Lp = Lp;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
@@ -846,6 +855,7 @@ int bwd_entry(const void* dout, const void* q, const void* k, const void* v, con
   p.trace = g_fab_trace; p.trace_cap = g_fab_trace_cap;
   p.dq = (bf16*)dq; p.dk = (bf16*)dk; p.dv = (bf16*)dv; p.err = g_fab_err[dev];
   p.kbias = kbias; p.Lkb = (Lk + T - 1) / T * T;
+  p.q_ld = ld.q; p.dq_ld = ld.dq; p.dk_ld = ld.dk; p.dv_ld = ld.dv;
   return DH == 128 ? launch_bwd<128>(tq, tk, tv, td, p, st) : launch_bwd<64>(tq, tk, tv, td, p, st);
 }
 
@@ -890,7 +900,15 @@ int eri_flash_attn_bwd_ld(const void* dout, const void* q, const void* k, const 
                           void* dk, void* dv, int B, int H, int Lq, int Lk, int DH, float scale,
                           long long out_ld, void* stream) {
   return bwd_entry(dout, q, k, v, out, lse, lse2, delta, dq, dk, dv, nullptr, B, H, Lq, Lk, DH, scale,
-                   stream, out_ld);
+                   stream, EriAttnStrides{0, 0, 0, out_ld, 0, 0, 0});
+}
+
+// Any of the operands but dout a column block of a wider matrix (attn_args.h); kbias may be null when Lk >= 128.
+int eri_flash_attn_bwd_strided(const void* dout, const void* q, const void* k, const void* v, const void* out,
+                               const float* lse, float* lse2, float* delta, void* dq, void* dk, void* dv,
+                               const float* kbias, int B, int H, int Lq, int Lk, int DH, float scale,
+                               const EriAttnStrides* ld, void* stream) {
+  return bwd_entry(dout, q, k, v, out, lse, lse2, delta, dq, dk, dv, kbias, B, H, Lq, Lk, DH, scale, stream, *ld);
 }
 
 // The same with the additive key bias of eri_flash_attn_fwd_masked (the forward's lse already
@@ -1028,6 +1046,7 @@ int eri_flash_attn_bwd_noalloc(const void* dout, const void* q, const void* k, c
   p.trace = g_fab_trace; p.trace_cap = g_fab_trace_cap;
   p.dq = (bf16*)dq; p.dk = (bf16*)dk; p.dv = (bf16*)dv; p.err = g_fa_noalloc_status_addr[dev];
   p.kbias = nullptr; p.Lkb = 0;
+  p.q_ld = p.dq_ld = p.dk_ld = p.dv_ld = (long long)H * DH;
   return DH == 128 ? launch_bwd<128>(tq, tk, tv, td, p, st) : launch_bwd<64>(tq, tk, tv, td, p, st);
 }
 

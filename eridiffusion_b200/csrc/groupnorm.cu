@@ -26,8 +26,12 @@ struct GnArgs {
   const bf16 *x, *dy, *w, *b;
   float *mean, *rstd;        // [N, G]
   float* part;               // [N, chunks, G, 2] group records
-  float* part_c;             // [N, chunks, C, 2] channel records (backward)
+  float* part_c;             // [N, chunks, C, 2 or 3] channel records (backward; sum xhat last, with pre only)
   bf16 *out, *dw, *db;
+  // x + pre_c[c] + pre_nc[n, c] is what gets normalised (either may be null): the bias of the convolution that
+  // produced x and a per-sample embedding, added here instead of in passes of their own
+  const bf16 *pre_c, *pre_nc;
+  bf16 *dpre_c, *dpre_nc;    // their gradients: sums of dx
   int N, HW, C, G, silu, chunks, rows_per_chunk, accumulate, apply_ctas;
   int gchunks;               // group records per sample that the apply pass adds (1 after a fold)
   float eps;
@@ -56,16 +60,31 @@ __device__ __forceinline__ void fold_groups(const GnArgs& a, int n, float* s) {
   __syncthreads();
 }
 
-template <bool BWD>
+// The per-channel addend of x for eight channels.
+__device__ __forceinline__ void load_pre(const GnArgs& a, int n, int v, float (&pr)[8]) {
+  float t[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) pr[j] = 0.f;
+  if (a.pre_c) unpack8(reinterpret_cast<const bf16x8*>(a.pre_c)[v], pr);
+  if (a.pre_nc) {
+    unpack8(reinterpret_cast<const bf16x8*>(a.pre_nc + (size_t)n * a.C)[v], t);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) pr[j] += t[j];
+  }
+}
+
+template <bool BWD, bool PRE>
 __global__ void __launch_bounds__(kMaxThreads) gn_column_kernel(const GnArgs a) {
-  extern __shared__ float sm[];     // [R][C][2] partial sums of the CTA's row lanes
+  constexpr int S = BWD && PRE ? 3 : 2;
+  extern __shared__ float sm[];     // [R][C][S] partial sums of the CTA's row lanes
   const int n = blockIdx.y, nvec = a.C >> 3;
   const int R = blockDim.x / nvec;
   const int v = threadIdx.x % nvec, rr = threadIdx.x / nvec;
   const int r0 = blockIdx.x * a.rows_per_chunk, r1 = min(a.HW, r0 + a.rows_per_chunk);
-  float s0[8], s1[8];
+  float s0[8], s1[8], s2[8], pr[8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) s0[j] = s1[j] = 0.f;
+  for (int j = 0; j < 8; ++j) s0[j] = s1[j] = s2[j] = pr[j] = 0.f;
+  if (PRE && rr < R) load_pre(a, n, v, pr);
   const bf16x8* xp = reinterpret_cast<const bf16x8*>(a.x + (size_t)n * a.HW * a.C) + v;
   if (rr < R) {
     if constexpr (!BWD) {
@@ -81,6 +100,7 @@ __global__ void __launch_bounds__(kMaxThreads) gn_column_kernel(const GnArgs a) 
             unpack8(q[u], f);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
+              if (PRE) f[j] += pr[j];
               s0[j] += f[j];
               s1[j] = fmaf(f[j], f[j], s1[j]);
             }
@@ -100,7 +120,7 @@ __global__ void __launch_bounds__(kMaxThreads) gn_column_kernel(const GnArgs a) 
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int g = (v * 8 + j) / cpg;
-        mu[j] = a.mean[n * a.G + g];
+        mu[j] = a.mean[n * a.G + g] - pr[j];
         rs[j] = a.rstd[n * a.G + g];
       }
       for (int r = r0 + rr; r < r1; r += R * 2) {
@@ -123,25 +143,27 @@ __global__ void __launch_bounds__(kMaxThreads) gn_column_kernel(const GnArgs a) 
               const float dz = a.silu ? g[j] * silu_grad_of(fmaf(xh, wv[j], bv[j])) : g[j];
               s0[j] += dz;
               s1[j] = fmaf(dz, xh, s1[j]);
+              if (PRE) s2[j] += xh;
             }
           }
       }
     }
-    float* o = sm + ((size_t)rr * a.C + v * 8) * 2;
+    float* o = sm + ((size_t)rr * a.C + v * 8) * S;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      o[2 * j] = s0[j];
-      o[2 * j + 1] = s1[j];
+      o[S * j] = s0[j];
+      o[S * j + 1] = s1[j];
+      if (S == 3) o[S * j + 2] = s2[j];
     }
   }
   __syncthreads();
   // row lanes -> one record per channel, in the first lane's slots
-  for (int i = threadIdx.x; i < 2 * a.C; i += blockDim.x) {
+  for (int i = threadIdx.x; i < S * a.C; i += blockDim.x) {
     float t = sm[i];
-    for (int r = 1; r < R; ++r) t += sm[(size_t)r * a.C * 2 + i];
+    for (int r = 1; r < R; ++r) t += sm[(size_t)r * a.C * S + i];
     if constexpr (BWD) {
-      a.part_c[((size_t)n * a.chunks + blockIdx.x) * a.C * 2 + i] = t;
-      t *= __bfloat162float(a.w[i >> 1]);
+      a.part_c[((size_t)n * a.chunks + blockIdx.x) * a.C * S + i] = t;
+      t *= __bfloat162float(a.w[i / S]);
     }
     sm[i] = t;
   }
@@ -151,7 +173,7 @@ __global__ void __launch_bounds__(kMaxThreads) gn_column_kernel(const GnArgs a) 
   for (int i = threadIdx.x; i < 2 * a.G; i += blockDim.x) {
     const int g = i >> 1;
     float t = 0.f;
-    for (int c = 0; c < cpg; ++c) t += sm[(g * cpg + c) * 2 + (i & 1)];
+    for (int c = 0; c < cpg; ++c) t += sm[(g * cpg + c) * S + (i & 1)];
     dst[i] = t;
   }
 }
@@ -176,29 +198,61 @@ __global__ void gn_fold_kernel(GnArgs a, float* folded) {
   }
 }
 
-template <bool BWD>
-__global__ void __launch_bounds__(kMaxThreads) gn_apply_kernel(const GnArgs a) {
-  extern __shared__ float sm[];     // [2 * G]
-  const int nvec = a.C >> 3;
-  if (BWD && (int)blockIdx.x >= a.apply_ctas) {
-    // parameter gradients: one warp-row of lanes per eight channels would be idle work for the apply CTAs
-    if (blockIdx.y) return;
-    const int cta = blockIdx.x - a.apply_ctas, per = blockDim.x / 8;     // eight record lanes per channel pair slot
-    const int i = cta * per + (int)threadIdx.x / 8, l = threadIdx.x & 7;   // i: index into [C][2]
-    float t = 0.f;
-    if (i < 2 * a.C) {
-      const int total = a.N * a.chunks;
-      for (int c = l; c < total; c += 8) t += a.part_c[(size_t)c * a.C * 2 + i];
-    }
+// Parameter gradients of 32 channels: eight lanes per channel over the chunk records of every sample.
+template <bool PRE>
+__device__ __forceinline__ void param_gradients(const GnArgs& a, int cta, float* sm) {
+  constexpr int S = PRE ? 3 : 2;
+  const int lanes = blockDim.x / 32, cl = threadIdx.x & 31, l = threadIdx.x >> 5, c = cta * 32 + cl;
+  const int cpg = a.C / a.G;
+  const float inv_m = 1.f / ((float)a.HW * (float)cpg);
+  float dw = 0.f, db = 0.f, dp = 0.f;
+  for (int n = 0; n < a.N; ++n) {
+    float t[3] = {0.f, 0.f, 0.f}, gs[2] = {0.f, 0.f};
+    if (c < a.C) {
+      for (int k = l; k < a.chunks; k += lanes) {
+        const float* p = a.part_c + (((size_t)n * a.chunks + k) * a.C + c) * S;
 #pragma unroll
-    for (int o = 4; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (i < 2 * a.C && l == 0) {
-      bf16* dst = (i & 1) ? a.dw : a.db;
-      if (dst) {
-        if (a.accumulate & ((i & 1) ? 1 : 2)) t += __bfloat162float(dst[i >> 1]);
-        dst[i >> 1] = __float2bfloat16(t);
+        for (int i = 0; i < S; ++i) t[i] += p[i];
+      }
+      if (PRE)
+        for (int k = l; k < a.gchunks; k += lanes) {
+          const float* p = a.part + (((size_t)n * a.gchunks + k) * a.G + c / cpg) * 2;
+          gs[0] += p[0];
+          gs[1] += p[1];
+        }
+    }
+    __syncthreads();
+    float* mine = sm + (l * 32 + cl) * 5;
+    mine[0] = t[0]; mine[1] = t[1]; mine[2] = t[2]; mine[3] = gs[0]; mine[4] = gs[1];
+    __syncthreads();
+    if (l == 0 && c < a.C) {
+      float r[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+      for (int k = 0; k < lanes; ++k)
+#pragma unroll
+        for (int i = 0; i < 5; ++i) r[i] += sm[(k * 32 + cl) * 5 + i];
+      db += r[0];
+      dw += r[1];
+      if (PRE) {
+        // sum over the rows of dx = rstd * (dz * w - s1 - xhat * s2)
+        const float d = a.rstd[n * a.G + c / cpg] * (__bfloat162float(a.w[c]) * r[0] - (float)a.HW * r[3] * inv_m - r[4] * inv_m * r[2]);
+        dp += d;
+        if (a.dpre_nc) a.dpre_nc[(size_t)n * a.C + c] = __float2bfloat16(d);
       }
     }
+  }
+  if (l == 0 && c < a.C) {
+    if (a.dw) a.dw[c] = __float2bfloat16(dw + ((a.accumulate & 1) ? __bfloat162float(a.dw[c]) : 0.f));
+    if (a.db) a.db[c] = __float2bfloat16(db + ((a.accumulate & 2) ? __bfloat162float(a.db[c]) : 0.f));
+    if (a.dpre_c) a.dpre_c[c] = __float2bfloat16(dp + ((a.accumulate & 4) ? __bfloat162float(a.dpre_c[c]) : 0.f));
+  }
+}
+
+template <bool BWD, bool PRE>
+__global__ void __launch_bounds__(kMaxThreads) gn_apply_kernel(const GnArgs a) {
+  extern __shared__ float sm[];     // [2 * G]; parameter CTAs [threads / 32][32][5]
+  const int nvec = a.C >> 3;
+  if (BWD && (int)blockIdx.x >= a.apply_ctas) {
+    if (blockIdx.y == 0) param_gradients<PRE>(a, blockIdx.x - a.apply_ctas, sm);
     return;
   }
   const int n = blockIdx.y, cpg = a.C / a.G;
@@ -220,7 +274,7 @@ __global__ void __launch_bounds__(kMaxThreads) gn_apply_kernel(const GnArgs a) {
   const int R = blockDim.x / nvec;
   const int v = threadIdx.x % nvec, rr = threadIdx.x / nvec;
   if (rr >= R) return;
-  float wv[8], bv[8];
+  float wv[8], bv[8], pr[8];
   unpack8(reinterpret_cast<const bf16x8*>(a.w)[v], wv);
   if (a.b) {
     unpack8(reinterpret_cast<const bf16x8*>(a.b)[v], bv);
@@ -228,6 +282,7 @@ __global__ void __launch_bounds__(kMaxThreads) gn_apply_kernel(const GnArgs a) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) bv[j] = 0.f;
   }
+  if (PRE) load_pre(a, n, v, pr);
   const size_t base = (size_t)n * a.HW * nvec + v;
   const bf16x8* xp = reinterpret_cast<const bf16x8*>(a.x) + base;
   bf16x8* op = reinterpret_cast<bf16x8*>(a.out) + base;
@@ -237,7 +292,7 @@ __global__ void __launch_bounds__(kMaxThreads) gn_apply_kernel(const GnArgs a) {
     for (int j = 0; j < 8; ++j) {
       const int g = (v * 8 + j) / cpg;
       wv[j] *= sm[2 * g + 1];
-      bv[j] = fmaf(-sm[2 * g], wv[j], bv[j]);
+      bv[j] = fmaf((PRE ? pr[j] : 0.f) - sm[2 * g], wv[j], bv[j]);
     }
     for (int r = blockIdx.x * R + rr; r < a.HW; r += step * kUnroll) {
       bf16x8 q[kUnroll];
@@ -263,7 +318,7 @@ __global__ void __launch_bounds__(kMaxThreads) gn_apply_kernel(const GnArgs a) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int g = (v * 8 + j) / cpg;
-      mu[j] = a.mean[n * a.G + g];
+      mu[j] = a.mean[n * a.G + g] - (PRE ? pr[j] : 0.f);
       rs[j] = a.rstd[n * a.G + g];
       t1[j] = sm[2 * g] * inv_m;
       t2[j] = sm[2 * g + 1] * inv_m;
@@ -317,8 +372,8 @@ GnPlan plan_for(int N, int HW, int C) {
   return p;
 }
 
-template <bool BWD>
-int run(GnArgs a, float* ws, cudaStream_t st) {
+template <bool BWD, bool PRE>
+int run_v(GnArgs a, float* ws, cudaStream_t st) {
   const GnPlan p = plan_for(a.N, a.HW, a.C);
   if (p.threads > kMaxThreads || 2 * a.G > 1024) return -1;
   a.chunks = a.gchunks = p.chunks;
@@ -327,25 +382,34 @@ int run(GnArgs a, float* ws, cudaStream_t st) {
   a.part = ws;
   float* folded = ws + (size_t)a.N * p.chunks * a.G * 2;
   a.part_c = folded + (size_t)a.N * a.G * 2;
-  const int smem = p.R * a.C * 2 * (int)sizeof(float);
+  constexpr int S = BWD && PRE ? 3 : 2;
+  const int smem = p.R * a.C * S * (int)sizeof(float);
   static bool configured[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -2;
   if (!configured[dev]) {
-    if (cudaFuncSetAttribute(gn_column_kernel<BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536) != cudaSuccess)
+    if (cudaFuncSetAttribute(gn_column_kernel<BWD, PRE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kMaxThreads * 8 * S * (int)sizeof(float)) != cudaSuccess)
       return -2;
     configured[dev] = true;
   }
-  gn_column_kernel<BWD><<<dim3(p.chunks, a.N), p.threads, smem, st>>>(a);
+  gn_column_kernel<BWD, PRE><<<dim3(p.chunks, a.N), p.threads, smem, st>>>(a);
   if (p.chunks > kMaxDirectChunks) {
     const int lanes = 1024 / (2 * a.G) < 1 ? 1 : 1024 / (2 * a.G);
     gn_fold_kernel<<<a.N, lanes * 2 * a.G, lanes * 2 * a.G * sizeof(float), st>>>(a, folded);
     a.part = folded;
     a.gchunks = 1;
   }
-  const int extra = BWD && (a.dw || a.db) ? (2 * a.C + p.threads / 8 - 1) / (p.threads / 8) : 0;
-  gn_apply_kernel<BWD><<<dim3(p.apply_ctas + extra, a.N), p.threads, 2 * a.G * sizeof(float), st>>>(a);
+  const bool params = BWD && (a.dw || a.db || a.dpre_c || a.dpre_nc);
+  const int extra = params ? (a.C + 31) / 32 : 0;
+  int smem_apply = 2 * a.G * (int)sizeof(float);
+  if (params && p.threads * 5 * (int)sizeof(float) > smem_apply) smem_apply = p.threads * 5 * (int)sizeof(float);
+  gn_apply_kernel<BWD, PRE><<<dim3(p.apply_ctas + extra, a.N), p.threads, smem_apply, st>>>(a);
   return (int)cudaGetLastError();
+}
+template <bool BWD>
+int run(const GnArgs& a, float* ws, cudaStream_t st) {
+  return a.pre_c || a.pre_nc ? run_v<BWD, true>(a, ws, st) : run_v<BWD, false>(a, ws, st);
 }
 
 }  // namespace
@@ -355,27 +419,32 @@ extern "C" {
 // fp32 words of workspace one call needs.
 long long eri_gn_workspace(int N, int HW, int C, int G, int backward) {
   const GnPlan p = plan_for(N, HW, C);
-  return (long long)N * (p.chunks + 1) * G * 2 + (backward ? (long long)N * p.chunks * C * 2 : 0);
+  return (long long)N * (p.chunks + 1) * G * 2 + (backward ? (long long)N * p.chunks * C * 3 : 0);
 }
 
-// y = act(GroupNorm(x)); mean / rstd [N, G] are written for the backward when given.
-int eri_gn_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, float* ws, int N, int HW,
-               int C, int G, float eps, int silu, void* stream) {
+// y = act(GroupNorm(x + pre_c + pre_nc)); mean / rstd [N, G] are written for the backward when given. pre_c [C] and
+// pre_nc [N, C] (bf16) may be null.
+int eri_gn_fwd(const void* x, const void* pre_c, const void* pre_nc, const void* w, const void* b, void* y, float* mean,
+               float* rstd, float* ws, int N, int HW, int C, int G, float eps, int silu, void* stream) {
   if (C % 8 || C % G) return -1;
   GnArgs a = {};
   a.x = (const bf16*)x; a.w = (const bf16*)w; a.b = (const bf16*)b; a.out = (bf16*)y; a.mean = mean; a.rstd = rstd;
+  a.pre_c = (const bf16*)pre_c; a.pre_nc = (const bf16*)pre_nc;
   a.N = N; a.HW = HW; a.C = C; a.G = G; a.silu = silu; a.eps = eps;
   return run<false>(a, ws, (cudaStream_t)stream);
 }
 
-// dx, and the parameter gradients dw / db [C] (bf16; null: not wanted). accumulate: bit 0 adds into dw, bit 1 into db.
-int eri_gn_bwd(const void* x, const void* dy, const void* w, const void* b, const float* mean, const float* rstd, void* dx,
-               void* dw, void* db, float* ws, int N, int HW, int C, int G, int silu, int accumulate, void* stream) {
+// dx, the parameter gradients dw / db [C] and those of pre_c / pre_nc (bf16; null: not wanted). accumulate: bit 0 adds
+// into dw, bit 1 into db, bit 2 into dpre_c.
+int eri_gn_bwd(const void* x, const void* pre_c, const void* pre_nc, const void* dy, const void* w, const void* b,
+               const float* mean, const float* rstd, void* dx, void* dw, void* db, void* dpre_c, void* dpre_nc, float* ws,
+               int N, int HW, int C, int G, int silu, int accumulate, void* stream) {
   if (C % 8 || C % G) return -1;
   GnArgs a = {};
   a.x = (const bf16*)x; a.dy = (const bf16*)dy; a.w = (const bf16*)w; a.b = (const bf16*)b;
+  a.pre_c = (const bf16*)pre_c; a.pre_nc = (const bf16*)pre_nc;
   a.mean = const_cast<float*>(mean); a.rstd = const_cast<float*>(rstd);
-  a.out = (bf16*)dx; a.dw = (bf16*)dw; a.db = (bf16*)db;
+  a.out = (bf16*)dx; a.dw = (bf16*)dw; a.db = (bf16*)db; a.dpre_c = (bf16*)dpre_c; a.dpre_nc = (bf16*)dpre_nc;
   a.N = N; a.HW = HW; a.C = C; a.G = G; a.silu = silu; a.accumulate = accumulate;
   return run<true>(a, ws, (cudaStream_t)stream);
 }

@@ -398,60 +398,67 @@ Tensor pad_bias(int64_t B, int64_t Lk, const Tensor& like) {
 
 }  // namespace
 
+namespace {
+
+// Token stride of a [B, L, H, D] operand the kernels read or write in place (heads packed).
+int64_t token_stride(const Tensor& t) {
+  const int64_t ld = t.stride(1), H = t.size(2), D = t.size(3);
+  const bool ok = t.stride(3) == 1 && t.stride(2) == D && ld >= H * D && ld % 8 == 0 && al16(t) &&
+                  (t.size(0) == 1 || t.stride(0) == t.size(1) * ld);
+  return ok ? ld : 0;
+}
+Tensor packed_heads(const Tensor& t) { return token_stride(t) ? t : t.contiguous(); }
+
+}  // namespace
+
 std::pair<Tensor, Tensor> attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, double scale, const Tensor& out_,
                                    const Tensor& kbias, int pair_poly) {
   const int64_t B = q.size(0), Lq = q.size(1), H = q.size(2), D = q.size(3), Lk = k.size(1);
-  Tensor out = out_.defined() ? out_ : at::empty_like(q);
-  int64_t ld = 0;
-  if (!out.is_contiguous()) {
-    ld = out.stride(1);
-    TORCH_CHECK_VALUE(out.stride(3) == 1 && out.stride(2) == D && ld >= H * D && ld % 8 == 0 &&
-                          (B == 1 || out.stride(0) == Lq * ld),
-                      "flash attention: unsupported output strides");
-    TORCH_CHECK_VALUE(!kbias.defined(), "flash attention: a strided output is not supported together with a key bias");
-  }
+  Tensor out = out_.defined() ? out_ : empty_bf16({B, Lq, H, D}, q);
+  EriAttnStrides ld = {};
+  ld.q = token_stride(q); ld.k = token_stride(k); ld.v = token_stride(v); ld.out = token_stride(out);
+  TORCH_CHECK_VALUE(ld.q && ld.k && ld.v && ld.out, "flash attention: unsupported operand strides");
   Tensor lse = empty_f32({B, H, Lq}, q);
-  if (kbias.defined()) {
-    check(L.eri_flash_attn_fwd_masked(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), (float*)lse.data_ptr(),
-                                      (const float*)kbias.data_ptr(), (int)B, (int)H, (int)Lq, (int)Lk, (int)D, (float)scale,
-                                      stream()), "flash_attn_fwd_masked");
-    return {out, lse};
-  }
-  if (pair_poly >= 0 && !ld && D == 128 && Lq >= 256 && Lk >= 128) {
+  if (pair_poly >= 0 && !kbias.defined() && out.is_contiguous() && q.is_contiguous() && k.is_contiguous() &&
+      v.is_contiguous() && D == 128 && Lq >= 256 && Lk >= 128) {
     const int code = L.eri_flash_attn_fwd_pair(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), (float*)lse.data_ptr(),
                                                (int)B, (int)H, (int)Lq, (int)Lk, (int)D, (float)scale, pair_poly, stream());
     if (code != -100) return check(code, "flash_attn_fwd_pair"), std::pair<Tensor, Tensor>{out, lse};
   }
-  check(L.eri_flash_attn_fwd_ld(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), (float*)lse.data_ptr(), (int)B,
-                                (int)H, (int)Lq, (int)Lk, (int)D, (float)scale, ld, stream()), "flash_attn_fwd");
+  check(L.eri_flash_attn_fwd_strided(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), (float*)lse.data_ptr(),
+                                     (const float*)ptr(kbias), (int)B, (int)H, (int)Lq, (int)Lk, (int)D, (float)scale, &ld,
+                                     stream()), "flash_attn_fwd");
   return {out, lse};
+}
+
+// dq, dk, dv: where the gradients go (heads packed, any token stride).
+void attn_bwd_into(const Tensor& dout, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& out, const Tensor& lse,
+                   double scale, const Tensor& kbias, const Tensor& dq, const Tensor& dk, const Tensor& dv) {
+  const int64_t B = q.size(0), Lq = q.size(1), H = q.size(2), D = q.size(3), Lk = k.size(1), Lp = (Lq + 127) / 128 * 128;
+  Tensor aux = empty_f32({2, B, H, Lp}, q);
+  float *lse2 = (float*)aux.data_ptr(), *delta = lse2 + B * H * Lp;
+  EriAttnStrides ld = {};
+  ld.q = token_stride(q); ld.k = token_stride(k); ld.v = token_stride(v); ld.out = token_stride(out);
+  ld.dq = token_stride(dq); ld.dk = token_stride(dk); ld.dv = token_stride(dv);
+  check(L.eri_flash_attn_bwd_strided(dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
+                                     (const float*)lse.data_ptr(), lse2, delta, dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+                                     (const float*)ptr(kbias), (int)B, (int)H, (int)Lq, (int)Lk, (int)D, (float)scale, &ld,
+                                     stream()), "flash_attn_bwd");
 }
 
 std::tuple<Tensor, Tensor, Tensor> attn_bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const Tensor& v,
                                             const Tensor& out, const Tensor& lse, double scale, const Tensor& kbias) {
-  const int64_t B = q.size(0), Lq = q.size(1), H = q.size(2), D = q.size(3), Lk = k.size(1), Lp = (Lq + 127) / 128 * 128;
-  Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v);
-  Tensor aux = empty_f32({2, B, H, Lp}, q);
-  float *lse2 = (float*)aux.data_ptr(), *delta = lse2 + B * H * Lp;
-  if (kbias.defined())
-    check(L.eri_flash_attn_bwd_masked(dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
-                                      (const float*)lse.data_ptr(), lse2, delta, dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
-                                      (const float*)kbias.data_ptr(), (int)B, (int)H, (int)Lq, (int)Lk, (int)D, (float)scale,
-                                      stream()), "flash_attn_bwd_masked");
-  else
-    check(L.eri_flash_attn_bwd_ld(dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
-                                  (const float*)lse.data_ptr(), lse2, delta, dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), (int)B,
-                                  (int)H, (int)Lq, (int)Lk, (int)D, (float)scale, out.is_contiguous() ? 0 : out.stride(1),
-                                  stream()), "flash_attn_bwd");
+  Tensor dq = empty_bf16(q.sizes(), q), dk = empty_bf16(k.sizes(), k), dv = empty_bf16(v.sizes(), v);
+  attn_bwd_into(dout, q, k, v, out, lse, scale, kbias, dq, dk, dv);
   return {dq, dk, dv};
 }
 
 namespace {
+
 struct Attention : torch::autograd::Function<Attention> {
-  static Tensor forward(AutogradContext* ctx, const OptT& q_o, const OptT& k_o, const OptT& v_o, const OptT& kbias_o,
-                        double scale, int64_t pair_poly) {
-    const Tensor q = opt(q_o), k = opt(k_o), v = opt(v_o), kbias = opt(kbias_o);
-    if (ctx) ctx->saved_data["args"] = Args({&q, &k, &v, &kbias}).mask;
+  static Tensor forward(AutogradContext* ctx, const OptT& q_o, const OptT& k_o, const OptT& v_o, const OptT& kbias_o, double scale,
+                        int64_t pair_poly) {
+    const Tensor q = packed_heads(*q_o), k = packed_heads(*k_o), v = packed_heads(*v_o), kbias = opt(kbias_o);
     auto [out, lse] = attn_fwd(q, k, v, scale, Tensor(), kbias, (int)pair_poly);
     ctx->save_for_backward({q, k, v, out, lse, kbias});
     ctx->saved_data["s"] = scale;
@@ -463,14 +470,73 @@ struct Attention : torch::autograd::Function<Attention> {
     return {dq, dk, dv, Tensor(), Tensor(), Tensor()};
   }
 };
+
+// Attention whose operands are column blocks of projections' outputs, read in place; the gradients are written as the
+// column blocks of the projections' output gradients. ``kv`` undefined: q, k and v are all in ``a`` [B, L, 3 * H * D]
+// (self-attention); else a = q [B, L, H * D] and kv [B, Lk, 2 * H * D]. Neither direction has a split, concatenation
+// or copy of its own.
+struct Parts {
+  Tensor q, k, v;
+  Parts(const Tensor& a, const Tensor& kv, int64_t H) {
+    const int64_t B = a.size(0), Lq = a.size(1);
+    if (kv.defined()) {
+      const int64_t D = a.size(2) / H;
+      Tensor s = kv.view({B, kv.size(1), 2, H, D});
+      q = a.view({B, Lq, H, D});
+      k = s.select(2, 0);
+      v = s.select(2, 1);
+    } else {
+      Tensor s = a.view({B, Lq, 3, H, a.size(2) / (3 * H)});
+      q = s.select(2, 0);
+      k = s.select(2, 1);
+      v = s.select(2, 2);
+    }
+  }
+};
+struct PackedAttention : torch::autograd::Function<PackedAttention> {
+  static Tensor forward(AutogradContext* ctx, const OptT& a_o, const OptT& kv_o, const OptT& kbias_o, int64_t heads, double scale) {
+    const Tensor a = contig(opt(a_o)), kv = contig(opt(kv_o)), kbias = opt(kbias_o);
+    Parts p(a, kv, heads);
+    auto [out, lse] = attn_fwd(p.q, p.k, p.v, scale, Tensor(), kbias, -1);
+    ctx->save_for_backward({a, kv, out, lse, kbias});
+    ctx->saved_data["s"] = scale;
+    ctx->saved_data["h"] = heads;
+    return out.flatten(2);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    auto sv = ctx->get_saved_variables();
+    const int64_t heads = ctx->saved_data["h"].toInt();
+    Tensor da = empty_bf16(sv[0].sizes(), sv[0]), dkv;
+    if (sv[1].defined()) dkv = empty_bf16(sv[1].sizes(), sv[1]);
+    Parts p(sv[0], sv[1], heads), d(da, dkv, heads);
+    attn_bwd_into(contig(g[0]), p.q, p.k, p.v, sv[2], sv[3], ctx->saved_data["s"].toDouble(), sv[4], d.q, d.k, d.v);
+    return {da, dkv, Tensor(), Tensor(), Tensor()};
+  }
+};
+
+Tensor packed_attention(const Tensor& a, const Tensor& kv, int64_t heads, double scale, const OptT& kbias_) {
+  Tensor kbias = opt(kbias_);
+  const int64_t Lk = kv.defined() ? kv.size(1) : a.size(1);
+  if (!kbias.defined() && Lk < 128) kbias = pad_bias(a.size(0), Lk, a);
+  if (any_grad({&a, &kv})) return PackedAttention::apply(wrap(a), wrap(kv), wrap(kbias), heads, scale);
+  Parts p(contig(a), contig(kv), heads);
+  return attn_fwd(p.q, p.k, p.v, scale, Tensor(), kbias, -1).first.flatten(2);
+}
+
 }  // namespace
 
-// q, k, v [B, L, H, Dh] contiguous; kbias from flash_attn.key_bias or none. pair_poly < 0: one-CTA forward.
+// q, k, v [B, L, H, Dh]; kbias from flash_attn.key_bias or none. pair_poly < 0: one-CTA forward.
 Tensor attention(const Tensor& q, const Tensor& k, const Tensor& v, double scale, const OptT& kbias_, int pair_poly) {
   Tensor kbias = opt(kbias_);
   if (!kbias.defined() && k.size(1) < 128) kbias = pad_bias(k.size(0), k.size(1), q);
   if (any_grad({&q, &k, &v})) return Attention::apply(wrap(q), wrap(k), wrap(v), wrap(kbias), scale, (int64_t)pair_poly);
-  return attn_fwd(q, k, v, scale, Tensor(), kbias, pair_poly).first;
+  return attn_fwd(packed_heads(q), packed_heads(k), packed_heads(v), scale, Tensor(), kbias, pair_poly).first;
+}
+Tensor attention_qkv(const Tensor& qkv, int64_t heads, double scale, const OptT& kbias) {
+  return packed_attention(qkv, Tensor(), heads, scale, kbias);
+}
+Tensor attention_kv(const Tensor& q, const Tensor& kv, int64_t heads, double scale, const OptT& kbias) {
+  return packed_attention(q, kv, heads, scale, kbias);
 }
 
 // ---------------------------------------------------------------------------------------------------- loss
@@ -498,53 +564,139 @@ Tensor mse_loss(const Tensor& pred, const Tensor& target, const OptT& weight) {
   return MseLoss::apply(wrap(pred), wrap(target), weight);
 }
 
-// ----------------------------------------------------------------------------------------- GroupNorm (+SiLU)
+// ------------------------------------------------------------------------ channels-last convolution helpers
+// Activations are [N, HW, C] rows or [N, C, H, W] in channels-last format (the same memory); results keep the form.
 namespace {
-Tensor gn_forward(const Tensor& x, const Tensor& w, const Tensor& b, int64_t groups, double eps, bool silu, Tensor& stats) {
-  const int N = (int)x.size(0), HW = (int)x.size(1), C = (int)x.size(2);
-  Tensor y = at::empty_like(x), ws = empty_f32({L.eri_gn_workspace(N, HW, C, (int)groups, 0)}, x);
+
+struct Rows {
+  int N, HW, C;
+  explicit Rows(const Tensor& x) {
+    N = (int)x.size(0);
+    C = (int)(x.dim() == 4 ? x.size(1) : x.size(2));
+    HW = (int)(x.dim() == 4 ? x.size(2) * x.size(3) : x.size(1));
+  }
+};
+Tensor rows_contig(const Tensor& x) {
+  return x.dim() == 4 ? x.contiguous(at::MemoryFormat::ChannelsLast) : contig(x);
+}
+
+// GroupNorm (+SiLU) of x + pre_c + pre_nc: the bias of the convolution before it and a per-sample embedding are added
+// where x is read.
+Tensor gn_forward(const Tensor& x, const Tensor& w, const Tensor& b, const Tensor& pc, const Tensor& pn, int64_t groups,
+                  double eps, bool silu, const Tensor& stats) {
+  const Rows r(x);
+  Tensor y = at::empty_like(x), ws = empty_f32({L.eri_gn_workspace(r.N, r.HW, r.C, (int)groups, 0)}, x);
   float* st = stats.defined() ? (float*)stats.data_ptr() : nullptr;
-  check(L.eri_gn_fwd(x.data_ptr(), w.data_ptr(), ptr(b), y.data_ptr(), st, st ? st + N * groups : nullptr, (float*)ws.data_ptr(), N,
-                     HW, C, (int)groups, (float)eps, silu, stream()), "gn_fwd");
+  check(L.eri_gn_fwd(x.data_ptr(), ptr(pc), ptr(pn), w.data_ptr(), ptr(b), y.data_ptr(), st, st ? st + r.N * groups : nullptr,
+                     (float*)ws.data_ptr(), r.N, r.HW, r.C, (int)groups, (float)eps, silu, stream()), "gn_fwd");
   return y;
 }
 struct GroupNormSilu : torch::autograd::Function<GroupNormSilu> {
-  static Tensor forward(AutogradContext* ctx, const OptT& x__o, const OptT& w_o, const OptT& b_o, int64_t groups, double eps,
-                        bool silu) {
-    const Tensor x_ = opt(x__o), w = opt(w_o), b = opt(b_o);
-    if (ctx) ctx->saved_data["args"] = Args({&x_, &w, &b}).mask;
-    Tensor x = contig(x_), stats = empty_f32({2, x.size(0), groups}, x);
-    Tensor y = gn_forward(x, w, b, groups, eps, silu, stats);
-    ctx->save_for_backward({x, w, b, stats});
+  static Tensor forward(AutogradContext* ctx, const OptT& x_o, const OptT& w_o, const OptT& b_o, const OptT& pc_o,
+                        const OptT& pn_o, int64_t groups, double eps, bool silu) {
+    const Tensor x = rows_contig(*x_o), w = *w_o, b = opt(b_o), pc = opt(pc_o), pn = contig(opt(pn_o));
+    ctx->saved_data["args"] = Args({&x, &w, &b, &pc, &pn}).mask;
+    Tensor stats = empty_f32({2, x.size(0), groups}, x);
+    Tensor y = gn_forward(x, w, b, pc, pn, groups, eps, silu, stats);
+    ctx->save_for_backward({x, w, b, stats, pc, pn});
     ctx->saved_data["m"] = std::vector<int64_t>{groups, silu};
     return y;
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     auto sv = ctx->get_saved_variables();
-    const Tensor &x = sv[0], &w = sv[1], &b = sv[2], &stats = sv[3];
+    const Tensor &x = sv[0], &w = sv[1], &b = sv[2], &stats = sv[3], &pc = sv[4], &pn = sv[5];
     const auto m = ctx->saved_data["m"].toIntVector();
-    const int N = (int)x.size(0), HW = (int)x.size(1), C = (int)x.size(2), G = (int)m[0];
-    Tensor dy = contig(g[0]), dx = at::empty_like(x), ws = empty_f32({L.eri_gn_workspace(N, HW, C, G, 1)}, x);
+    const int G = (int)m[0];
+    const Rows r(x);
+    Tensor dy = rows_contig(g[0]), dx = at::empty_like(x), ws = empty_f32({L.eri_gn_workspace(r.N, r.HW, r.C, G, 1)}, x);
     const Args args(ctx->saved_data["args"].toInt());
-    const bool nw = args.need(ctx, 1), nb = args.need(ctx, 2);
-    const bool aw = nw && has_grad_buffer(w, at::kBFloat16), ab = nb && has_grad_buffer(b, at::kBFloat16);
-    Tensor rw, rb;
-    if (nw && !aw) rw = empty_bf16({C}, x);
-    if (nb && !ab) rb = empty_bf16({C}, x);
+    // a parameter's gradient goes straight into its buffer when it has one
+    variable_list out(8);
+    int acc = 0;
+    auto dest = [&](int arg, const Tensor& p, int bit) -> void* {
+      if (!args.need(ctx, arg)) return nullptr;
+      if (has_grad_buffer(p, at::kBFloat16)) {
+        acc |= bit;
+        return p.grad().data_ptr();
+      }
+      out[arg] = empty_bf16({r.C}, x);
+      return out[arg].data_ptr();
+    };
+    void *dw = dest(1, w, 1), *db = dest(2, b, 2), *dpc = dest(3, pc, 4), *dpn = nullptr;
+    if (args.need(ctx, 4)) {
+      out[4] = empty_bf16({r.N, r.C}, x);
+      dpn = out[4].data_ptr();
+    }
     const float* st = (const float*)stats.data_ptr();
-    check(L.eri_gn_bwd(x.data_ptr(), dy.data_ptr(), w.data_ptr(), ptr(b), st, st + N * G, dx.data_ptr(),
-                       aw ? w.grad().data_ptr() : mptr(rw), ab ? b.grad().data_ptr() : mptr(rb), (float*)ws.data_ptr(), N, HW, C, G,
-                       (int)m[1], (aw ? 1 : 0) | (ab ? 2 : 0), stream()), "gn_bwd");
-    return {dx, rw, rb, Tensor(), Tensor(), Tensor()};
+    check(L.eri_gn_bwd(x.data_ptr(), ptr(pc), ptr(pn), dy.data_ptr(), w.data_ptr(), ptr(b), st, st + r.N * G, dx.data_ptr(), dw, db,
+                       dpc, dpn, (float*)ws.data_ptr(), r.N, r.HW, r.C, G, (int)m[1], acc, stream()), "gn_bwd");
+    out[0] = dx;
+    return out;
   }
 };
+
+Tensor add_bias_forward(const Tensor& a, const Tensor& b, const Tensor& bias, const Tensor& bias2) {
+  const Rows r(a);
+  Tensor out = at::empty_like(a);
+  check(L.eri_add_bias(a.data_ptr(), b.data_ptr(), ptr(bias), ptr(bias2), out.data_ptr(), (long long)r.N * r.HW, r.C, stream()),
+        "add_bias");
+  return out;
+}
+// [N * HW, C] view of a channels-last activation
+Tensor as_matrix(const Tensor& x) {
+  const Rows r(x);
+  return x.dim() == 4 ? x.permute({0, 2, 3, 1}).view({(int64_t)r.N * r.HW, r.C}) : x.view({(int64_t)r.N * r.HW, r.C});
+}
+struct AddBias : torch::autograd::Function<AddBias> {
+  static Tensor forward(AutogradContext* ctx, const OptT& a_o, const OptT& b_o, const OptT& bias_o, const OptT& bias2_o) {
+    const Tensor a = rows_contig(*a_o), b = rows_contig(*b_o), bias = opt(bias_o), bias2 = opt(bias2_o);
+    ctx->saved_data["args"] = Args({&a, &b, &bias, &bias2}).mask;
+    ctx->save_for_backward({bias, bias2});
+    return add_bias_forward(a, b, bias, bias2);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    auto sv = ctx->get_saved_variables();
+    const Args args(ctx->saved_data["args"].toInt());
+    Tensor d = rows_contig(g[0]);
+    variable_list out{d, d, Tensor(), Tensor()};
+    for (int i = 0; i < 2; ++i)
+      if (args.need(ctx, 2 + i)) out[2 + i] = col_sum(as_matrix(d), sv[i]);
+    return out;
+  }
+};
+
+struct Upsample2x : torch::autograd::Function<Upsample2x> {
+  static Tensor run(const Tensor& x, bool backward) {
+    const int64_t N = x.size(0), C = x.size(1), H = backward ? x.size(2) / 2 : x.size(2), W = backward ? x.size(3) / 2 : x.size(3);
+    Tensor y = at::empty({N, C, backward ? H : 2 * H, backward ? W : 2 * W}, x.options(), at::MemoryFormat::ChannelsLast);
+    check(L.eri_upsample2x(x.data_ptr(), y.data_ptr(), N * H, (int)W, (int)C, backward, stream()), "upsample2x");
+    return y;
+  }
+  static Tensor forward(AutogradContext* ctx, const Tensor& x) { return run(rows_contig(x), false); }
+  static variable_list backward(AutogradContext* ctx, variable_list g) { return {run(rows_contig(g[0]), true)}; }
+};
+
 }  // namespace
 
-Tensor group_norm_silu(const Tensor& rows, const Tensor& w, const OptT& b_, int64_t groups, double eps, bool silu) {
-  Tensor b = opt(b_);
-  if (any_grad({&rows, &w, &b})) return GroupNormSilu::apply(wrap(rows), wrap(w), wrap(b), groups, eps, silu);
-  Tensor none;
-  return gn_forward(contig(rows), w, b, groups, eps, silu, none);
+Tensor group_norm_silu(const Tensor& x, const Tensor& w, const OptT& b_, const OptT& pc_, const OptT& pn_, int64_t groups,
+                       double eps, bool silu) {
+  Tensor b = opt(b_), pc = opt(pc_), pn = opt(pn_);
+  if (any_grad({&x, &w, &b, &pc, &pn}))
+    return GroupNormSilu::apply(wrap(x), wrap(w), wrap(b), wrap(pc), wrap(pn), groups, eps, silu);
+  return gn_forward(rows_contig(x), w, b, pc, contig(pn), groups, eps, silu, Tensor());
+}
+
+// a + b + bias + bias2 (per channel): a block's residual sum with the biases of its last convolutions.
+Tensor add_bias(const Tensor& a, const Tensor& b, const OptT& bias_, const OptT& bias2_) {
+  Tensor bias = opt(bias_), bias2 = opt(bias2_);
+  if (any_grad({&a, &b, &bias, &bias2})) return AddBias::apply(wrap(a), wrap(b), wrap(bias), wrap(bias2));
+  return add_bias_forward(rows_contig(a), rows_contig(b), bias, bias2);
+}
+
+// Nearest-neighbour upsampling by two of an [N, C, H, W] activation.
+Tensor upsample2x(const Tensor& x) {
+  if (any_grad({&x})) return Upsample2x::apply(x);
+  return Upsample2x::run(rows_contig(x), false);
 }
 
 // ------------------------------------------------------------------------------- FLUX single-stream block

@@ -14,6 +14,7 @@
 #include <tuple>
 #include <vector>
 
+#include "../attn_args.h"
 #include "../gemm_args.h"
 
 namespace eri_ops {
@@ -48,10 +49,12 @@ using torch::autograd::variable_list;
   X(eri_glu_fwd, (const void*, void*, int, int, int, int, void*))                                                \
   X(eri_glu_bwd, (const void*, const void*, void*, int, int, int, int, void*))                                   \
   X(eri_mse_fwd_bwd, (const void*, const void*, const float*, float*, void*, long long, long long, float, void*)) \
-  X(eri_gn_fwd, (const void*, const void*, const void*, void*, float*, float*, float*, int, int, int, int, float, \
-                 int, void*))                                                                                    \
-  X(eri_gn_bwd, (const void*, const void*, const void*, const void*, const float*, const float*, void*, void*,   \
-                 void*, float*, int, int, int, int, int, int, void*))                                            \
+  X(eri_gn_fwd, (const void*, const void*, const void*, const void*, const void*, void*, float*, float*, float*, \
+                 int, int, int, int, float, int, void*))                                                         \
+  X(eri_gn_bwd, (const void*, const void*, const void*, const void*, const void*, const void*, const float*,     \
+                 const float*, void*, void*, void*, void*, void*, float*, int, int, int, int, int, int, void*))  \
+  X(eri_add_bias, (const void*, const void*, const void*, const void*, void*, long long, int, void*))            \
+  X(eri_upsample2x, (const void*, void*, long long, int, int, int, void*))                                       \
   X(eri_gemm_skinny, (const void*, long long, const void*, long long, void*, int, int, int, int, float, void*))  \
   X(eri_gemm_rank_stream, (const void*, long long, const void*, long long, void*, int, int, int, int, float,     \
                            void*))                                                                               \
@@ -72,16 +75,11 @@ using torch::autograd::variable_list;
   X(eri_rows_wgrad, (const void*, int, const void*, int, void*, int, int, int, int, int, float, void*))          \
   X(eri_rows_dgrad, (const void*, int, const void*, int, float*, int, int, int, int, void*))                     \
   X(eri_gemv_bf16, (const void*, const void*, const void*, void*, int, int, int, int, int, int, int, int, void*)) \
-  X(eri_flash_attn_fwd_ld, (const void*, const void*, const void*, void*, float*, int, int, int, int, int,       \
-                            float, long long, void*))                                                            \
-  X(eri_flash_attn_fwd_masked, (const void*, const void*, const void*, void*, float*, const float*, int, int,    \
-                                int, int, int, float, void*))                                                    \
-  X(eri_flash_attn_bwd_ld, (const void*, const void*, const void*, const void*, const void*, const float*,       \
-                            float*, float*, void*, void*, void*, int, int, int, int, int, float, long long,      \
-                            void*))                                                                              \
-  X(eri_flash_attn_bwd_masked, (const void*, const void*, const void*, const void*, const void*, const float*,   \
-                                float*, float*, void*, void*, void*, const float*, int, int, int, int, int,      \
-                                float, void*))
+  X(eri_flash_attn_fwd_strided, (const void*, const void*, const void*, void*, float*, const float*, int, int,   \
+                                 int, int, int, float, const EriAttnStrides*, void*))                            \
+  X(eri_flash_attn_bwd_strided, (const void*, const void*, const void*, const void*, const void*, const float*,  \
+                                 float*, float*, void*, void*, void*, const float*, int, int, int, int, int,     \
+                                 float, const EriAttnStrides*, void*))
 
 struct Lib {
   long long (*eri_gn_workspace)(int, int, int, int, int) = nullptr;
@@ -173,8 +171,13 @@ Tensor act(const Tensor& x, int mode);
 Tensor glu(const Tensor& h, int mode, bool act_first);
 std::vector<Tensor> split_tokens(const Tensor& x, int64_t n);
 Tensor attention(const Tensor& q, const Tensor& k, const Tensor& v, double scale, const OptT& kbias, int pair_poly);
+Tensor attention_qkv(const Tensor& qkv, int64_t heads, double scale, const OptT& kbias);
+Tensor attention_kv(const Tensor& q, const Tensor& kv, int64_t heads, double scale, const OptT& kbias);
 Tensor mse_loss(const Tensor& pred, const Tensor& target, const OptT& weight);
-Tensor group_norm_silu(const Tensor& rows, const Tensor& weight, const OptT& bias, int64_t groups, double eps, bool silu);
+Tensor group_norm_silu(const Tensor& x, const Tensor& weight, const OptT& bias, const OptT& pre_c, const OptT& pre_nc,
+                       int64_t groups, double eps, bool silu);
+Tensor add_bias(const Tensor& a, const Tensor& b, const OptT& bias, const OptT& bias2);
+Tensor upsample2x(const Tensor& x);
 Tensor single_stream(const Tensor& xm, const Tensor& x, const Tensor& gate, const Tensor& w1, const OptT& b1,
                      const Tensor& w2, const OptT& b2, const OptT& a1, const OptT& bb1, double s1, const OptT& a2,
                      const OptT& bb2, double s2, const OptT& qs, const OptT& ks, const OptT& cos, const OptT& sin,

@@ -45,7 +45,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("glu", &glu);
   m.def("split_tokens", &split_tokens);
   m.def("attention", &attention);
+  m.def("attention_qkv", &attention_qkv);
+  m.def("attention_kv", &attention_kv);
   m.def("mse_loss", &mse_loss);
   m.def("group_norm_silu", &group_norm_silu);
+  m.def("add_bias", &add_bias);
+  m.def("upsample2x", &upsample2x);
   m.def("single_stream", &single_stream);
 }

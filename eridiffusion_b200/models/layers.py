@@ -117,6 +117,15 @@ def mlp_pair(up0, down0, x0, up1, down1, x1, act="gelu", residual=(None, None), 
 _MLP_FUSE = _os.environ.get("ERI_B200_MLP_FUSE", "0") == "1"
 
 
+def channels_last_convs(model):
+    """Keep every convolution weight in the memory order the channels-last kernels read, so that no call
+    converts it (29 MB for a 1280-channel 3x3 convolution, 10 us per call)."""
+    for m in model.modules():
+        if isinstance(m, nn.Conv2d):
+            m.weight.data = m.weight.data.contiguous(memory_format=torch.channels_last)
+    return model
+
+
 class SmallLinear(Linear):
     """Linear applied to a few conditioning rows (adaLN modulation, embedders)."""
 

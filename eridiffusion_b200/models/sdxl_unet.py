@@ -19,7 +19,7 @@ import torch.nn as nn
 import torch.nn.functional as TF
 
 from ..ops import functional as F
-from .layers import Linear, timestep_embedding
+from .layers import Linear, channels_last_convs, timestep_embedding
 from .registry import register_model
 
 
@@ -69,15 +69,11 @@ class CrossAttention(nn.Module):
         self.to_out = Linear(dim, dim, dtype=dtype, device=device)
 
     def forward(self, x, ctx=None, residual=None):
-        B, L, D = x.shape
-        H = self.heads
+        # the attention reads q, k and v inside the projections' outputs: no split or copy in either direction
         if self.self_attn:
-            q, k, v = F.qknorm_rope(self.to_qkv(x), None, None, None, None, H)
+            o = F.attention_qkv(self.to_qkv(x), self.heads)
         else:
-            q = self.to_q(x).view(B, L, H, D // H)
-            kv = self.to_kv(ctx).view(B, ctx.shape[1], 2, H, D // H)
-            k, v = kv[:, :, 0].contiguous(), kv[:, :, 1].contiguous()
-        o = F.attention(q, k, v).reshape(B, L, D)
+            o = F.attention_kv(self.to_q(x), self.to_kv(ctx), self.heads)
         return self.to_out(o, residual=residual)
 
 
@@ -108,8 +104,8 @@ class GroupNormAct(nn.GroupNorm):
         super().__init__(groups, ch, eps=eps, dtype=dtype, device=device)
         self.silu = silu
 
-    def forward(self, x):
-        return F.group_norm_silu(x, self.weight, self.bias, self.num_groups, self.eps, self.silu)
+    def forward(self, x, pre_c=None, pre_nc=None):
+        return F.group_norm_silu(x, self.weight, self.bias, self.num_groups, self.eps, self.silu, pre_c, pre_nc)
 
 
 class Transformer2D(nn.Module):
@@ -128,8 +124,8 @@ class Transformer2D(nn.Module):
         h = self.proj_in(h)
         for blk in self.blocks:
             h = blk(h, ctx)
-        h = self.proj_out(h)
-        return x + h.view(B, H, W, C).permute(0, 3, 1, 2)
+        h = self.proj_out(h, residual=x.permute(0, 2, 3, 1).reshape(B, H * W, C))
+        return h.view(B, H, W, C).permute(0, 3, 1, 2)
 
 
 class ResBlock(nn.Module):
@@ -143,6 +139,15 @@ class ResBlock(nn.Module):
         self.skip = nn.Conv2d(cin, cout, 1, dtype=dtype, device=device) if cin != cout else None
 
     def forward(self, x, emb):
+        if F.conv_fusable(x, self.conv1, self.conv2, self.skip):
+            # the first convolution's bias and the time embedding are added where the second norm reads its input,
+            # the other biases in the residual sum
+            h = F.conv_no_bias(self.conv1, self.norm1(x))
+            h = self.norm2(h, self.conv1.bias, F.small_linear(emb, self.temb.weight, self.temb.bias, silu_in=True))
+            h = F.conv_no_bias(self.conv2, h)
+            if self.skip is None:
+                return F.add_bias(x, h, self.conv2.bias)
+            return F.add_bias(F.conv_no_bias(self.skip, x), h, self.conv2.bias, self.skip.bias)
         h = self.conv1(self.norm1(x))                                       # GroupNorm + SiLU fused
         h = h + self.temb(TF.silu(emb))[:, :, None, None]
         h = self.conv2(self.norm2(h))
@@ -197,6 +202,7 @@ class SDXLUNet(nn.Module):
                 self.up_kinds.append("up")
         self.norm_out = GroupNormAct(cfg.groups, ch[0], 1e-5, True, **kw)
         self.conv_out = nn.Conv2d(ch[0], cfg.out_channels, 3, padding=1, **kw)
+        channels_last_convs(self)
 
     def conditioning(self, t, pooled, time_ids):
         """emb = time_mlp(sin(t)) + add_mlp([pooled | sin(time_ids)]) (2816 -> 1280)."""
@@ -244,7 +250,7 @@ class SDXLUNet(nn.Module):
             h = h + mid_res.to(h.dtype)
         for kind, m in zip(self.up_kinds, self.up):
             if kind == "up":
-                h = m(TF.interpolate(h, scale_factor=2.0, mode="nearest"))
+                h = m(F.upsample2x(h))
             else:
                 h = m[0](torch.cat([h, hs.pop()], dim=1), emb)
                 h = m[1](h, ctx) if not isinstance(m[1], nn.Identity) else h

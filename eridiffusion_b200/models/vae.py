@@ -17,6 +17,7 @@ import torch.nn as nn
 import torch.nn.functional as TF
 
 from ..ops import functional as F
+from .layers import channels_last_convs
 from .registry import register_model
 
 
@@ -46,8 +47,8 @@ class _GN(nn.GroupNorm):
         super().__init__(groups, ch, eps=1e-6, **kw)
         self.silu = silu
 
-    def forward(self, x):
-        return F.group_norm_silu(x, self.weight, self.bias, self.num_groups, self.eps, self.silu)
+    def forward(self, x, pre_c=None):
+        return F.group_norm_silu(x, self.weight, self.bias, self.num_groups, self.eps, self.silu, pre_c)
 
 
 class _Res(nn.Module):
@@ -58,6 +59,12 @@ class _Res(nn.Module):
         self.skip = nn.Conv2d(cin, cout, 1, **kw) if cin != cout else None
 
     def forward(self, x):
+        if F.conv_fusable(x, self.c1, self.c2, self.skip):
+            # the convolutions' biases are added where the second norm reads its input and in the residual sum
+            h = F.conv_no_bias(self.c2, self.n2(F.conv_no_bias(self.c1, self.n1(x)), self.c1.bias))
+            if self.skip is None:
+                return F.add_bias(x, h, self.c2.bias)
+            return F.add_bias(F.conv_no_bias(self.skip, x), h, self.c2.bias, self.skip.bias)
         h = self.c2(self.n2(self.c1(self.n1(x))))
         return (x if self.skip is None else self.skip(x)) + h
 
@@ -128,7 +135,7 @@ class Decoder(nn.Module):
         for b in self.mid:
             h = b(h)
         for b in self.up:
-            h = b(TF.interpolate(h, scale_factor=2.0, mode="nearest")) if isinstance(b, nn.Conv2d) else b(h)
+            h = b(F.upsample2x(h)) if isinstance(b, nn.Conv2d) else b(h)
         return self.conv_out(self.norm_out(h))
 
 
@@ -140,6 +147,7 @@ class AutoencoderKL(nn.Module):
         self.encoder, self.decoder = Encoder(cfg, kw), Decoder(cfg, kw)
         self.quant_conv = nn.Conv2d(2 * cfg.latent_channels, 2 * cfg.latent_channels, 1, **kw)
         self.post_quant_conv = nn.Conv2d(cfg.latent_channels, cfg.latent_channels, 1, **kw)
+        channels_last_convs(self)
 
     def moments(self, img):
         """img [B, 3, H, W] in [-1, 1] -> (mean, logvar) of the latent posterior."""

@@ -640,6 +640,39 @@ def attention(q, k, v, scale=None, mask=None, out=None):
     return R.attention(q, k, v, scale, mask)
 
 
+def _packed_ok(head_dim, mask, B, Lk, *ts) -> bool:
+    from . import flash_attn as FA
+    return (_ATTN_NATIVE == "native" and head_dim in (64, 128) and _native_ok(*ts) and ts[0].shape[1] >= 16 and FA.has_forward()
+            and (mask is None or FA.mask_is_key_only(mask, B, Lk)))
+
+
+def attention_qkv(qkv, num_heads, scale=None, mask=None):
+    """Self-attention on a packed projection [B, L, 3*H*Dh] -> [B, L, H*Dh]. On the native path q, k and v are read
+    in place and the gradient is written as one packed tensor."""
+    B, L, W = qkv.shape
+    Dh = W // (3 * num_heads)
+    if _packed_ok(Dh, mask, B, L, qkv):
+        from . import flash_attn as FA
+        ATTENTION_CALLS["native"] += 1
+        kb = None if mask is None else FA.key_bias(mask, B, L, qkv.device)
+        return N.ops().attention_qkv(qkv, num_heads, scale if scale is not None else 1.0 / math.sqrt(Dh), kb)
+    q, k, v = qkv.view(B, L, 3, num_heads, Dh).unbind(2)
+    return attention(q.contiguous(), k.contiguous(), v.contiguous(), scale, mask).reshape(B, L, W // 3)
+
+
+def attention_kv(q, kv, num_heads, scale=None, mask=None):
+    """Cross-attention of q [B, L, H*Dh] on a packed key / value projection [B, Lk, 2*H*Dh] -> [B, L, H*Dh]."""
+    B, L, W = q.shape
+    Lk, Dh = kv.shape[1], W // num_heads
+    if _packed_ok(Dh, mask, B, Lk, q, kv):
+        from . import flash_attn as FA
+        ATTENTION_CALLS["native"] += 1
+        kb = None if mask is None else FA.key_bias(mask, B, Lk, q.device)
+        return N.ops().attention_kv(q, kv, num_heads, scale if scale is not None else 1.0 / math.sqrt(Dh), kb)
+    k, v = kv.view(B, Lk, 2, num_heads, Dh).unbind(2)
+    return attention(q.view(B, L, num_heads, Dh), k.contiguous(), v.contiguous(), scale, mask).reshape(B, L, W)
+
+
 # ---------------------------------------------------------------------------- losses / noise
 def mse_loss(pred, target, weight=None):
     """mean(weight[b] * (pred - target)^2) with the gradient produced in the same pass."""
@@ -699,10 +732,14 @@ def sumsq(flat, out=None):
 
 
 # ---------------------------------------------------------------------------- GroupNorm (+SiLU)
-def group_norm_silu(x, weight, bias=None, groups=32, eps=1e-5, silu=True):
+def group_norm_silu(x, weight, bias=None, groups=32, eps=1e-5, silu=True, pre_c=None, pre_nc=None):
     """GroupNorm followed by an optional SiLU on a channels-last activation. ``x`` is either
     [N, HW, C] or an [N, C, H, W] tensor in ``torch.channels_last`` memory format (returned in the
-    same logical shape and format)."""
+    same logical shape and format). ``pre_c`` [C] and ``pre_nc`` [N, C] are added to x before the norm (the
+    bias of the convolution that produced x and a per-sample embedding), in the same pass on the native path."""
+    C = x.shape[1] if x.dim() == 4 else x.shape[-1]
+    if _native_ok(x, weight, bias, pre_c, pre_nc) and C % 8 == 0 and C % groups == 0 and C <= 5120 and groups <= 512:
+        return N.ops().group_norm_silu(x, weight, bias, pre_c, pre_nc, groups, eps, silu)
     nchw = x.dim() == 4
     if nchw:
         Nn, C, H, W = x.shape
@@ -712,14 +749,52 @@ def group_norm_silu(x, weight, bias=None, groups=32, eps=1e-5, silu=True):
         rows = rows.view(Nn, H * W, C)
     else:
         rows = x
-    C = rows.shape[-1]
-    if _native_ok(rows, weight, bias) and C % 8 == 0 and C % groups == 0 and C <= 5120 and groups <= 512:
-        y = N.ops().group_norm_silu(rows, weight, bias, groups, eps, silu)
-    else:
-        y = R.group_norm_silu(rows, weight, bias, groups, eps, silu)
+    if pre_c is not None:
+        rows = rows + pre_c
+    if pre_nc is not None:
+        rows = rows + pre_nc[:, None, :]
+    y = R.group_norm_silu(rows, weight, bias, groups, eps, silu)
     if nchw:
         return y.view(Nn, H, W, C).permute(0, 3, 1, 2)
     return y
+
+
+def add_bias(a, b, bias=None, bias2=None):
+    """``a + b`` plus per-channel biases: the residual sum of a convolutional block with the biases of its last
+    convolutions. [N, HW, C] or channels-last [N, C, H, W]."""
+    C = a.shape[1] if a.dim() == 4 else a.shape[-1]
+    if _native_ok(a, b, bias, bias2) and C % 8 == 0 and a.shape == b.shape:
+        return N.ops().add_bias(a, b, bias, bias2)
+    y = a + b
+    for t in (bias, bias2):
+        if t is not None:
+            y = y + (t[:, None, None] if a.dim() == 4 else t)
+    return y
+
+
+def upsample2x(x):
+    """Nearest-neighbour upsampling by two of an [N, C, H, W] activation (channels-last on the native path)."""
+    if _native_ok(x) and x.dim() == 4 and x.shape[1] % 8 == 0:
+        return N.ops().upsample2x(x)
+    return torch.nn.functional.interpolate(x, scale_factor=2.0, mode="nearest")
+
+
+def conv_fusable(x, *convs) -> bool:
+    """Whether the biases of ``convs`` may be added by the ops around them (``group_norm_silu``'s ``pre_c``,
+    ``add_bias``) instead of in a pass after each convolution: plain convolutions on the native path."""
+    return _native_ok(x) and all(c is None or (type(c) is torch.nn.Conv2d and not c._forward_hooks and not c._forward_pre_hooks
+                                               and c.padding_mode == "zeros" and c.out_channels % 8 == 0) for c in convs)
+
+
+def conv_no_bias(conv, x):
+    """``conv(x)`` without its bias. A 1x1 convolution runs as a linear on the pixel rows."""
+    w = conv.weight
+    if conv.kernel_size == (1, 1) and conv.stride == (1, 1) and conv.padding == (0, 0) and conv.groups == 1 \
+            and x.shape[1] % 8 == 0:
+        Nn, C, H, W = x.shape
+        rows = x.permute(0, 2, 3, 1).reshape(Nn, H * W, C)
+        return linear(rows, w.view(w.shape[0], C)).view(Nn, H, W, w.shape[0]).permute(0, 3, 1, 2)
+    return torch.nn.functional.conv2d(x, w, None, conv.stride, conv.padding, conv.dilation, conv.groups)
 
 
 # ---------------------------------------------------------------------------- token routing
