@@ -407,7 +407,7 @@ int64_t token_stride(const Tensor& t) {
                   (t.size(0) == 1 || t.stride(0) == t.size(1) * ld);
   return ok ? ld : 0;
 }
-Tensor packed_heads(const Tensor& t) { return token_stride(t) ? t : t.contiguous(); }
+Tensor packed_heads(const Tensor& t) { return token_stride(t) ? t : contig16(t); }
 
 }  // namespace
 
@@ -466,7 +466,7 @@ struct Attention : torch::autograd::Function<Attention> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     auto sv = ctx->get_saved_variables();
-    auto [dq, dk, dv] = attn_bwd(contig(g[0]), sv[0], sv[1], sv[2], sv[3], sv[4], ctx->saved_data["s"].toDouble(), sv[5]);
+    auto [dq, dk, dv] = attn_bwd(contig16(g[0]), sv[0], sv[1], sv[2], sv[3], sv[4], ctx->saved_data["s"].toDouble(), sv[5]);
     return {dq, dk, dv, Tensor(), Tensor(), Tensor()};
   }
 };
@@ -495,7 +495,7 @@ struct Parts {
 };
 struct PackedAttention : torch::autograd::Function<PackedAttention> {
   static Tensor forward(AutogradContext* ctx, const OptT& a_o, const OptT& kv_o, const OptT& kbias_o, int64_t heads, double scale) {
-    const Tensor a = contig(opt(a_o)), kv = contig(opt(kv_o)), kbias = opt(kbias_o);
+    const Tensor a = contig16(opt(a_o)), kv = contig16(opt(kv_o)), kbias = opt(kbias_o);
     Parts p(a, kv, heads);
     auto [out, lse] = attn_fwd(p.q, p.k, p.v, scale, Tensor(), kbias, -1);
     ctx->save_for_backward({a, kv, out, lse, kbias});
@@ -509,7 +509,7 @@ struct PackedAttention : torch::autograd::Function<PackedAttention> {
     Tensor da = empty_bf16(sv[0].sizes(), sv[0]), dkv;
     if (sv[1].defined()) dkv = empty_bf16(sv[1].sizes(), sv[1]);
     Parts p(sv[0], sv[1], heads), d(da, dkv, heads);
-    attn_bwd_into(contig(g[0]), p.q, p.k, p.v, sv[2], sv[3], ctx->saved_data["s"].toDouble(), sv[4], d.q, d.k, d.v);
+    attn_bwd_into(contig16(g[0]), p.q, p.k, p.v, sv[2], sv[3], ctx->saved_data["s"].toDouble(), sv[4], d.q, d.k, d.v);
     return {da, dkv, Tensor(), Tensor(), Tensor()};
   }
 };
@@ -519,7 +519,7 @@ Tensor packed_attention(const Tensor& a, const Tensor& kv, int64_t heads, double
   const int64_t Lk = kv.defined() ? kv.size(1) : a.size(1);
   if (!kbias.defined() && Lk < 128) kbias = pad_bias(a.size(0), Lk, a);
   if (any_grad({&a, &kv})) return PackedAttention::apply(wrap(a), wrap(kv), wrap(kbias), heads, scale);
-  Parts p(contig(a), contig(kv), heads);
+  Parts p(contig16(a), contig16(kv), heads);
   return attn_fwd(p.q, p.k, p.v, scale, Tensor(), kbias, -1).first.flatten(2);
 }
 
@@ -537,6 +537,67 @@ Tensor attention_qkv(const Tensor& qkv, int64_t heads, double scale, const OptT&
 }
 Tensor attention_kv(const Tensor& q, const Tensor& kv, int64_t heads, double scale, const OptT& kbias) {
   return packed_attention(q, kv, heads, scale, kbias);
+}
+
+// Self-attention of a packed projection whose queries and keys are first normalised (RMS over the whole width) and
+// rotated: attention(rope(norm(q) * wq), rope(norm(k) * wk), v). q, k, v are read and their gradients written inside
+// the packed tensors.
+namespace {
+
+// fp32 table the kernels can read in 16-byte words
+Tensor rope_rows(const Tensor& t) {
+  Tensor f = t.to(at::kFloat);
+  return f.stride(1) == 1 && f.stride(0) % 4 == 0 && al16(f) ? f : contig16(f);
+}
+
+struct RopeAttention : torch::autograd::Function<RopeAttention> {
+  static Tensor forward(AutogradContext* ctx, const OptT& qkv_o, const OptT& wq_o, const OptT& wk_o, const OptT& cos_o,
+                        const OptT& sin_o, int64_t heads, double eps, bool keep) {
+    const Tensor qkv = contig16(*qkv_o), wq = contig16(*wq_o), wk = contig16(*wk_o);
+    const int64_t B = qkv.size(0), Lq = qkv.size(1), D = qkv.size(2) / 3;
+    Tensor cos = rope_rows(*cos_o), sin = rope_rows(*sin_o);
+    if (cos.stride(0) != sin.stride(0)) {
+      cos = contig16(cos);
+      sin = contig16(sin);
+    }
+    Parts p(qkv, Tensor(), heads);
+    Tensor q = empty_bf16({B, Lq, heads, D / heads}, qkv), k = at::empty_like(q), rstd = empty_f32({2, B * Lq}, qkv);
+    check(L.eri_norm_rope_fwd(p.q.data_ptr(), p.k.data_ptr(), 3 * D, wq.data_ptr(), wk.data_ptr(), (const float*)cos.data_ptr(),
+                              (const float*)sin.data_ptr(), cos.stride(0), q.data_ptr(), k.data_ptr(), (float*)rstd.data_ptr(),
+                              (int)(B * Lq), (int)Lq, (int)D, (float)eps, stream()), "norm_rope_fwd");
+    Tensor kbias = Lq < 128 ? pad_bias(B, Lq, qkv) : Tensor();
+    auto [out, lse] = attn_fwd(q, k, p.v, 1.0 / std::sqrt((double)(D / heads)), Tensor(), kbias, -1);
+    if (keep) {
+      ctx->save_for_backward({qkv, wq, wk, cos, sin, rstd, q, k, out, lse, kbias});
+      ctx->saved_data["h"] = heads;
+    }
+    return out.flatten(2);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    auto sv = ctx->get_saved_variables();
+    const Tensor &qkv = sv[0], &wq = sv[1], &wk = sv[2], &cos = sv[3], &sin = sv[4], &rstd = sv[5], &q = sv[6], &k = sv[7];
+    const int64_t heads = ctx->saved_data["h"].toInt(), B = q.size(0), Lq = q.size(1), D = q.size(2) * q.size(3);
+    Tensor d_qkv = empty_bf16(qkv.sizes(), qkv), dq = at::empty_like(q), dk = at::empty_like(k);
+    Parts p(qkv, Tensor(), heads), d(d_qkv, Tensor(), heads);
+    attn_bwd_into(contig16(g[0]), q, k, p.v, sv[8], sv[9], 1.0 / std::sqrt((double)(D / heads)), sv[10], dq, dk, d.v);
+    check(L.eri_norm_rope_bwd(p.q.data_ptr(), p.k.data_ptr(), 3 * D, wq.data_ptr(), wk.data_ptr(), (const float*)cos.data_ptr(),
+                              (const float*)sin.data_ptr(), cos.stride(0), (const float*)rstd.data_ptr(), dq.data_ptr(),
+                              dk.data_ptr(), d.q.data_ptr(), d.k.data_ptr(), 3 * D, (int)(B * Lq), (int)Lq, (int)D, stream()),
+          "norm_rope_bwd");
+    return {d_qkv, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+}  // namespace
+
+// wq, wk [D] and the tables [L, D / 2] get no gradient (the caller keeps to the separate ops where they need one).
+Tensor attention_qkv_rope(const Tensor& qkv, const Tensor& wq, const Tensor& wk, const Tensor& cos, const Tensor& sin,
+                          int64_t heads, double eps) {
+  const int64_t D = qkv.size(2) / 3;
+  TORCH_CHECK_VALUE(wq.numel() == D && wk.numel() == D && cos.dim() == 2 && cos.size(0) == qkv.size(1) && cos.size(1) * 2 == D &&
+                        sin.sizes() == cos.sizes(), "attention_qkv_rope: operand sizes");
+  if (any_grad({&qkv})) return RopeAttention::apply(wrap(qkv), wrap(wq), wrap(wk), wrap(cos), wrap(sin), heads, eps, true);
+  return RopeAttention::forward(nullptr, qkv, wq, wk, cos, sin, heads, eps, false);
 }
 
 // ---------------------------------------------------------------------------------------------------- loss
@@ -577,7 +638,8 @@ struct Rows {
   }
 };
 Tensor rows_contig(const Tensor& x) {
-  return x.dim() == 4 ? x.contiguous(at::MemoryFormat::ChannelsLast) : contig(x);
+  Tensor c = x.dim() == 4 ? x.contiguous(at::MemoryFormat::ChannelsLast) : contig(x);
+  return al16(c) ? c : c.clone();      // (a clone keeps the memory format)
 }
 
 // GroupNorm (+SiLU) of x + pre_c + pre_nc: the bias of the convolution before it and a per-sample embedding are added
@@ -594,7 +656,7 @@ Tensor gn_forward(const Tensor& x, const Tensor& w, const Tensor& b, const Tenso
 struct GroupNormSilu : torch::autograd::Function<GroupNormSilu> {
   static Tensor forward(AutogradContext* ctx, const OptT& x_o, const OptT& w_o, const OptT& b_o, const OptT& pc_o,
                         const OptT& pn_o, int64_t groups, double eps, bool silu) {
-    const Tensor x = rows_contig(*x_o), w = *w_o, b = opt(b_o), pc = opt(pc_o), pn = contig(opt(pn_o));
+    const Tensor x = rows_contig(*x_o), w = contig16(*w_o), b = contig16(opt(b_o)), pc = contig16(opt(pc_o)), pn = contig16(opt(pn_o));
     ctx->saved_data["args"] = Args({&x, &w, &b, &pc, &pn}).mask;
     Tensor stats = empty_f32({2, x.size(0), groups}, x);
     Tensor y = gn_forward(x, w, b, pc, pn, groups, eps, silu, stats);
@@ -649,7 +711,7 @@ Tensor as_matrix(const Tensor& x) {
 }
 struct AddBias : torch::autograd::Function<AddBias> {
   static Tensor forward(AutogradContext* ctx, const OptT& a_o, const OptT& b_o, const OptT& bias_o, const OptT& bias2_o) {
-    const Tensor a = rows_contig(*a_o), b = rows_contig(*b_o), bias = opt(bias_o), bias2 = opt(bias2_o);
+    const Tensor a = rows_contig(*a_o), b = rows_contig(*b_o), bias = contig16(opt(bias_o)), bias2 = contig16(opt(bias2_o));
     ctx->saved_data["args"] = Args({&a, &b, &bias, &bias2}).mask;
     ctx->save_for_backward({bias, bias2});
     return add_bias_forward(a, b, bias, bias2);
@@ -683,14 +745,14 @@ Tensor group_norm_silu(const Tensor& x, const Tensor& w, const OptT& b_, const O
   Tensor b = opt(b_), pc = opt(pc_), pn = opt(pn_);
   if (any_grad({&x, &w, &b, &pc, &pn}))
     return GroupNormSilu::apply(wrap(x), wrap(w), wrap(b), wrap(pc), wrap(pn), groups, eps, silu);
-  return gn_forward(rows_contig(x), w, b, pc, contig(pn), groups, eps, silu, Tensor());
+  return gn_forward(rows_contig(x), contig16(w), contig16(b), contig16(pc), contig16(pn), groups, eps, silu, Tensor());
 }
 
 // a + b + bias + bias2 (per channel): a block's residual sum with the biases of its last convolutions.
 Tensor add_bias(const Tensor& a, const Tensor& b, const OptT& bias_, const OptT& bias2_) {
   Tensor bias = opt(bias_), bias2 = opt(bias2_);
   if (any_grad({&a, &b, &bias, &bias2})) return AddBias::apply(wrap(a), wrap(b), wrap(bias), wrap(bias2));
-  return add_bias_forward(rows_contig(a), rows_contig(b), bias, bias2);
+  return add_bias_forward(rows_contig(a), rows_contig(b), contig16(bias), contig16(bias2));
 }
 
 // Nearest-neighbour upsampling by two of an [N, C, H, W] activation.

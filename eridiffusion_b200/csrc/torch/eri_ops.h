@@ -75,6 +75,11 @@ using torch::autograd::variable_list;
   X(eri_rows_wgrad, (const void*, int, const void*, int, void*, int, int, int, int, int, float, void*))          \
   X(eri_rows_dgrad, (const void*, int, const void*, int, float*, int, int, int, int, void*))                     \
   X(eri_gemv_bf16, (const void*, const void*, const void*, void*, int, int, int, int, int, int, int, int, void*)) \
+  X(eri_norm_rope_fwd, (const void*, const void*, long long, const void*, const void*, const float*, const float*, \
+                        long long, void*, void*, float*, int, int, int, float, void*))                           \
+  X(eri_norm_rope_bwd, (const void*, const void*, long long, const void*, const void*, const float*, const float*, \
+                        long long, const float*, const void*, const void*, void*, void*, long long, int, int, int, \
+                        void*))                                                                                  \
   X(eri_flash_attn_fwd_strided, (const void*, const void*, const void*, void*, float*, const float*, int, int,   \
                                  int, int, int, float, const EriAttnStrides*, void*))                            \
   X(eri_flash_attn_bwd_strided, (const void*, const void*, const void*, const void*, const void*, const float*,  \
@@ -104,6 +109,12 @@ inline void* mptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr
 inline Tensor opt(const OptT& t) { return t.has_value() ? *t : Tensor(); }
 inline Tensor contig(const Tensor& t) { return !t.defined() || t.is_contiguous() ? t : t.contiguous(); }
 inline bool al16(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
+// contiguous and on a 16-byte boundary (a contiguous slice may start anywhere)
+inline Tensor contig16(const Tensor& t) {
+  if (!t.defined()) return t;
+  Tensor c = contig(t);
+  return al16(c) ? c : c.clone();
+}
 // bytes from t's first element to the end of its storage (what a kernel may touch through its pointer)
 inline long long extent(const Tensor& t) {
   return t.defined() ? (long long)t.storage().nbytes() - t.storage_offset() * (long long)t.element_size() : 0;
@@ -173,6 +184,8 @@ std::vector<Tensor> split_tokens(const Tensor& x, int64_t n);
 Tensor attention(const Tensor& q, const Tensor& k, const Tensor& v, double scale, const OptT& kbias, int pair_poly);
 Tensor attention_qkv(const Tensor& qkv, int64_t heads, double scale, const OptT& kbias);
 Tensor attention_kv(const Tensor& q, const Tensor& kv, int64_t heads, double scale, const OptT& kbias);
+Tensor attention_qkv_rope(const Tensor& qkv, const Tensor& wq, const Tensor& wk, const Tensor& cos, const Tensor& sin,
+                          int64_t heads, double eps);
 Tensor mse_loss(const Tensor& pred, const Tensor& target, const OptT& weight);
 Tensor group_norm_silu(const Tensor& x, const Tensor& weight, const OptT& bias, const OptT& pre_c, const OptT& pre_nc,
                        int64_t groups, double eps, bool silu);

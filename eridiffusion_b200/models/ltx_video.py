@@ -92,18 +92,18 @@ class LTXBlock(nn.Module):
     def _self_attention_local(self, h, cos, sin):
         B, L, D = h.shape
         qkv = self.attn1_qkv(h)
+        cp = getattr(self, "context_parallel", None)
+        if cp is None:
+            return F.attention_qkv_rope(qkv, self.attn1_qnorm, self.attn1_knorm, cos, sin, self.heads)
+        # tokens are sharded over the group; keys / values travel around the ring
+        from ..parallel.ring_attention import ring_attention
         q, k, v = qkv.split(D, dim=-1)
         q = F.norm_modulate(q.contiguous(), weight=self.attn1_qnorm, rms=True)
         k = F.norm_modulate(k.contiguous(), weight=self.attn1_knorm, rms=True)
         q, k = _rope_full(q, cos, sin), _rope_full(k, cos, sin)
         sh = (B, L, self.heads, D // self.heads)
-        cp = getattr(self, "context_parallel", None)
-        if cp is not None:
-            # tokens are sharded over the group; keys / values travel around the ring
-            from ..parallel.ring_attention import ring_attention
-            return ring_attention(q.view(sh).contiguous(), k.view(sh).contiguous(), v.contiguous().view(sh),
-                                  group=cp.group).view(B, L, D)
-        return F.attention(q.view(sh), k.view(sh), v.contiguous().view(sh)).view(B, L, D)
+        return ring_attention(q.view(sh).contiguous(), k.view(sh).contiguous(), v.contiguous().view(sh),
+                              group=cp.group).view(B, L, D)
 
     def _self_attention_ulysses(self, h, cos, sin, u, eps=1e-6):
         from ..parallel.ulysses import dist_rmsnorm, ulysses_qkv

@@ -673,6 +673,24 @@ def attention_kv(q, kv, num_heads, scale=None, mask=None):
     return attention(q.view(B, L, num_heads, Dh), k.contiguous(), v.contiguous(), scale, mask).reshape(B, L, W)
 
 
+def attention_qkv_rope(qkv, q_weight, k_weight, cos, sin, num_heads, eps=1e-6):
+    """Self-attention on a packed projection [B, L, 3*H*Dh] whose queries and keys are first normalised (RMS over all
+    H*Dh channels, times ``q_weight`` / ``k_weight``) and rotated over interleaved pairs of the whole width (cos / sin
+    [L, H*Dh/2]) -> [B, L, H*Dh]. One kernel reads q, k and the tables once; trainable norm weights use the separate ops."""
+    B, L, W = qkv.shape
+    D = W // 3
+    if _packed_ok(D // num_heads, None, B, L, qkv, q_weight, k_weight) and D % 8 == 0 and D <= 8192 and cos.is_cuda and sin.is_cuda \
+            and cos.shape == sin.shape == (L, D // 2) \
+            and not (torch.is_grad_enabled() and any(t.requires_grad for t in (q_weight, k_weight, cos, sin))):
+        ATTENTION_CALLS["native"] += 1
+        return N.ops().attention_qkv_rope(qkv, q_weight, k_weight, cos, sin, num_heads, eps)
+    q, k, v = qkv.split(D, dim=-1)
+    sh = (B, L, num_heads, D // num_heads)
+    q, k = (R.rope_rotate(norm_modulate(t.contiguous(), weight=w, rms=True, eps=eps).unsqueeze(2), cos, sin).squeeze(2).to(t.dtype)
+            for t, w in ((q, q_weight), (k, k_weight)))
+    return attention(q.view(sh), k.view(sh), v.contiguous().view(sh)).reshape(B, L, D)
+
+
 # ---------------------------------------------------------------------------- losses / noise
 def mse_loss(pred, target, weight=None):
     """mean(weight[b] * (pred - target)^2) with the gradient produced in the same pass."""
