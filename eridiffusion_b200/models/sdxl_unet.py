@@ -256,6 +256,15 @@ class SDXLUNet(nn.Module):
                 h = m[1](h, ctx) if not isinstance(m[1], nn.Identity) else h
         return self.conv_out(self.norm_out(h))
 
+    def samples_independent(self) -> bool:
+        """Whether two batches may share one call: no hooks, and every cross-attention is the model's own (an image
+        adapter's holds the tokens of one batch)."""
+        if self._forward_hooks or self._forward_pre_hooks:
+            return False
+        blocks = [b for m in (*self.down, self.mid, *self.up) if isinstance(m, nn.ModuleList)
+                  for t in m if isinstance(t, Transformer2D) for b in t.blocks]
+        return all(type(b) is BasicTransformerBlock and type(b.attn2) is CrossAttention for b in blocks)
+
     def lora_targets(self):
         return [r"\.attn[12]\.(to_qkv|to_q|to_kv|to_out)$", r"\.ff_(in|out)$"]
 

@@ -196,6 +196,22 @@ def generate_video_flow(model, txt, frames: int, height: int, width: int, channe
 _K_SAMPLERS = {"euler": sample_euler, "heun": sample_heun, "dpmpp_2m": sample_dpmpp_2m}
 
 
+# Latent pixels of the joint guidance batch: four images of 1024 x 1024. Above it the UNet's products fill the GPU by
+# themselves and joining the two predictions only doubles the activations.
+_JOINT_GUIDANCE_PIXELS = 4 * 128 * 128
+
+
+def _joint_guidance(model, ctx, neg_ctx, pooled, neg_pooled, height, width) -> bool:
+    """Whether the conditional and the unconditional prediction are made in one call of twice the batch. At batch 1 the
+    UNet's products have 1024-4096 rows, which leave most SMs idle, and its 1200 launches cost as much host time as the
+    device needs for them (two steps at 1024 x 1024: 78.9 ms apart, 54.9 ms joined); rows of a batch do not interact, so
+    the values are those of two calls."""
+    return (torch.is_tensor(pooled) and torch.is_tensor(neg_pooled) and ctx.shape == neg_ctx.shape
+            and pooled.shape == neg_pooled.shape and ctx.dtype == neg_ctx.dtype and pooled.dtype == neg_pooled.dtype
+            and 2 * ctx.shape[0] * (height // 8) * (width // 8) <= _JOINT_GUIDANCE_PIXELS
+            and getattr(model, "samples_independent", bool)())
+
+
 class UnifiedInferencePipeline:
     """One ``generate`` for every family. ``model`` is the denoiser (already on its device),
     ``vae`` an optional ``AutoencoderKL`` for decoding, ``text_encode`` an optional callable
@@ -271,8 +287,13 @@ class UnifiedInferencePipeline:
         if scale != 1.0:
             zc = torch.zeros_like(ctx) if neg_ctx is None else neg_ctx
             zp = torch.zeros_like(pooled) if neg_pooled is None else neg_pooled
-            den_u, cond = eps_denoiser(lambda x, t: m(x, t, zc, zp, tid), train_sigmas), den
-            den = lambda x, s: cfg_mix(cond(x, s), den_u(x, s), scale)
+            if _joint_guidance(m, ctx, zc, pooled, zp, height, width):
+                both = [torch.cat(p) for p in ((ctx, zc), (pooled, zp), (tid, tid))]
+                den2 = eps_denoiser(lambda x, t: m(x, t, *both), train_sigmas)
+                den = lambda x, s: cfg_mix(*den2(torch.cat((x, x)), s).chunk(2), scale)
+            else:
+                den_u, cond = eps_denoiser(lambda x, t: m(x, t, zc, zp, tid), train_sigmas), den
+                den = lambda x, s: cfg_mix(cond(x, s), den_u(x, s), scale)
         sig = karras_sigmas(steps, device=dev)
         gen = torch.Generator(device=dev).manual_seed(seed)
         x = torch.randn(B, 4, height // 8, width // 8, device=dev, generator=gen).to(dt) * sig[0]
