@@ -539,6 +539,21 @@ Tensor attention_kv(const Tensor& q, const Tensor& kv, int64_t heads, double sca
   return packed_attention(q, kv, heads, scale, kbias);
 }
 
+// q, k, v [B, L, H, 512] (column blocks of wider tensors are read in place), no gradient.
+Tensor attention_wide(const Tensor& q_, const Tensor& k_, const Tensor& v_, double scale) {
+  const Tensor q = packed_heads(q_), k = packed_heads(k_), v = packed_heads(v_);
+  const int64_t B = q.size(0), Lq = q.size(1), H = q.size(2), Lk = k.size(1);
+  TORCH_CHECK_VALUE(q.size(3) == 512 && k.sizes() == v.sizes() && k.size(0) == B && k.size(2) == H && k.size(3) == 512,
+                    "attention_wide: operand sizes");
+  Tensor out = empty_bf16({B, Lq, H, 512}, q);
+  EriAttnStrides ld = {};
+  ld.q = token_stride(q); ld.k = token_stride(k); ld.v = token_stride(v);
+  TORCH_CHECK_VALUE(ld.q && ld.k && ld.v, "attention_wide: unsupported operand strides");
+  check(L.eri_flash_attn_wide_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), (int)B, (int)H, (int)Lq, (int)Lk,
+                                  (float)scale, &ld, stream()), "flash_attn_wide");
+  return out;
+}
+
 // Self-attention of a packed projection whose queries and keys are first normalised (RMS over the whole width) and
 // rotated: attention(rope(norm(q) * wq), rope(norm(k) * wk), v). q, k, v are read and their gradients written inside
 // the packed tensors.

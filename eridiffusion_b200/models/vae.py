@@ -82,7 +82,7 @@ class _Attn(nn.Module):
         B, C, H, W = x.shape
         t = self.norm(x).permute(0, 2, 3, 1).reshape(B, H * W, C)
         q, k, v = self.qkv(t).view(B, H * W, 3, 1, C).unbind(2)
-        o = F.attention(q.contiguous(), k.contiguous(), v.contiguous()).reshape(B, H * W, C)
+        o = F.attention(q, k, v).reshape(B, H * W, C)      # read inside the projection's output
         return x + self.out(o).view(B, H, W, C).permute(0, 3, 1, 2)
 
 

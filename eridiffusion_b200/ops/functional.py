@@ -619,6 +619,9 @@ def attention(q, k, v, scale=None, mask=None, out=None):
         if FA.supported(q, k, v) and (mask is None or FA.mask_is_key_only(mask, q.shape[0], k.shape[1])):
             ATTENTION_CALLS["native"] += 1
             return FA.flash_attention(q, k, v, scale, out, mask)
+        if mask is None and out is None and _wide_ok(q, k, v):
+            ATTENTION_CALLS["native"] += 1
+            return N.ops().attention_wide(q, k, v, scale if scale is not None else 1.0 / math.sqrt(512))
         # other head sizes below 128 (SD1.5: 40 and 80) ride on the 64 / 128 kernels with zero columns
         # appended: zero query / key columns leave the scores unchanged, zero value columns give zero
         # output columns that are cut off again (the pad and the slice are differentiable copies)
@@ -638,6 +641,12 @@ def attention(q, k, v, scale=None, mask=None, out=None):
         if o is not None:
             return o
     return R.attention(q, k, v, scale, mask)
+
+
+def _wide_ok(q, k, v) -> bool:
+    """Head size 512 (the image autoencoders' middle block), forward only: tiles of 128 queries and 128 keys."""
+    return (q.shape[-1] == 512 and q.shape[1] >= 128 and k.shape[1] >= 128 and k.shape == v.shape and q.shape[0] == k.shape[0]
+            and q.shape[2] == k.shape[2] and not (torch.is_grad_enabled() and any(t.requires_grad for t in (q, k, v))))
 
 
 def _packed_ok(head_dim, mask, B, Lk, *ts) -> bool:
