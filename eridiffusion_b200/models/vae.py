@@ -58,15 +58,39 @@ class _Res(nn.Module):
         self.n2, self.c2 = _GN(groups, cout, True, kw), nn.Conv2d(cout, cout, 3, padding=1, **kw)
         self.skip = nn.Conv2d(cin, cout, 1, **kw) if cin != cout else None
 
-    def forward(self, x):
-        if F.conv_fusable(x, self.c1, self.c2, self.skip):
-            # the convolutions' biases are added where the second norm reads its input and in the residual sum
-            h = F.conv_no_bias(self.c2, self.n2(F.conv_no_bias(self.c1, self.n1(x)), self.c1.bias))
+    def fusable(self, x):
+        return F.conv_fusable(x, self.c1, self.c2, self.skip)
+
+    def forward(self, x, pre=None):
+        """``pre`` (with ``fusable`` only): the bias [C] of the convolution that produced x, not added yet."""
+        if self.fusable(x):
+            # the convolutions' biases are added where a norm reads its input and in the residual sum
+            h = F.conv_no_bias(self.c2, self.n2(F.conv_no_bias(self.c1, self.n1(x, pre)), self.c1.bias))
             if self.skip is None:
-                return F.add_bias(x, h, self.c2.bias)
-            return F.add_bias(F.conv_no_bias(self.skip, x), h, self.c2.bias, self.skip.bias)
+                return F.add_bias(x, h, self.c2.bias, pre)
+            sb = self.skip.bias if pre is None else F.small_linear(pre[None], self.skip.weight.flatten(1), self.skip.bias)[0]
+            return F.add_bias(F.conv_no_bias(self.skip, x), h, self.c2.bias, sb)
         h = self.c2(self.n2(self.c1(self.n1(x))))
         return (x if self.skip is None else self.skip(x)) + h
+
+
+def _run(blocks, h, resample, conv_in=None):
+    """Residual blocks and resampling convolutions in order. The bias of a convolution in front of a residual block is
+    added where that block reads its input instead of in a pass of its own (1.0 of 14 ms of a 1024 x 1024 decode)."""
+    pre, blocks = None, list(blocks)
+    if conv_in is not None:
+        blocks.insert(0, conv_in)
+    for i, b in enumerate(blocks):
+        if not isinstance(b, nn.Conv2d):
+            h, pre = (b(h) if pre is None else b(h, pre)), None
+            continue
+        h = h if b is conv_in else resample(h)
+        nxt = blocks[i + 1] if i + 1 < len(blocks) else None
+        if type(nxt) is _Res and b.bias is not None and F.conv_fusable(h, b) and nxt.fusable(h):
+            h, pre = F.conv_no_bias(b, h), b.bias
+        else:
+            h = b(h)
+    return h
 
 
 class _Attn(nn.Module):
@@ -104,9 +128,7 @@ class Encoder(nn.Module):
         self.conv_out = nn.Conv2d(c, 2 * cfg.latent_channels, 3, padding=1, **kw)
 
     def forward(self, x):
-        h = self.conv_in(x.contiguous(memory_format=torch.channels_last))
-        for b in self.down:
-            h = b(TF.pad(h, (0, 1, 0, 1))) if isinstance(b, nn.Conv2d) else b(h)
+        h = _run(self.down, x.contiguous(memory_format=torch.channels_last), lambda t: TF.pad(t, (0, 1, 0, 1)), self.conv_in)
         for b in self.mid:
             h = b(h)
         return self.conv_out(self.norm_out(h))
@@ -131,11 +153,8 @@ class Decoder(nn.Module):
         self.conv_out = nn.Conv2d(c, cfg.in_channels, 3, padding=1, **kw)
 
     def forward(self, z):
-        h = self.conv_in(z.contiguous(memory_format=torch.channels_last))
-        for b in self.mid:
-            h = b(h)
-        for b in self.up:
-            h = b(F.upsample2x(h)) if isinstance(b, nn.Conv2d) else b(h)
+        h = _run(self.mid, z.contiguous(memory_format=torch.channels_last), None, self.conv_in)
+        h = _run(self.up, h, F.upsample2x)
         return self.conv_out(self.norm_out(h))
 
 
