@@ -175,13 +175,26 @@ class DDPM:
             betas = rescale_zero_terminal_snr(betas)
         self.betas = betas
         self.alphas_cumprod = torch.cumprod(1.0 - betas, 0).clamp(1e-8, 0.999).float()
+        self._on_device = {}
 
     def sample_t(self, n, gen=None, device="cpu"):
         return torch.randint(0, self.num_steps, (n,), generator=gen, device=device)
 
     def _ab(self, t):
         idx = t.round().long().clamp(0, self.num_steps - 1)
-        return self.alphas_cumprod.to(t.device)[idx]
+        return self._table(t.device)[idx]
+
+    def _table(self, device):
+        """``alphas_cumprod`` on ``device``, copied there once: a copy from pageable host memory waits for the device,
+        which kept the host from preparing the next training step while the last one ran."""
+        src = self.alphas_cumprod
+        if src.device == device:
+            return src
+        made_from, version, table = self._on_device.get(device, (None, 0, None))
+        if made_from is not src or version != src._version:
+            table = src.to(device)
+            self._on_device[device] = (src, src._version, table)
+        return table
 
     def coefficients(self, t):
         ab = self._ab(t)
