@@ -554,6 +554,26 @@ Tensor attention_wide(const Tensor& q_, const Tensor& k_, const Tensor& v_, doub
   return out;
 }
 
+// q, k, v [B, L, H, 64 | 128] (column blocks of wider tensors are read in place) with an additive bf16 or boolean mask
+// that broadcasts to [B, H, Lq, Lk]; no gradient.
+Tensor attention_bias(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& bias, double scale) {
+  const Tensor q = packed_heads(q_), k = packed_heads(k_), v = packed_heads(v_);
+  const int64_t B = q.size(0), Lq = q.size(1), H = q.size(2), D = q.size(3), Lk = k.size(1);
+  const bool is_bool = bias.scalar_type() == at::kBool;
+  TORCH_CHECK_VALUE(k.sizes() == v.sizes() && k.size(0) == B && k.size(2) == H && k.size(3) == D && bias.device() == q.device() &&
+                        (is_bool || bias.scalar_type() == at::kBFloat16) && bias.dim() == 4 && bias.size(3) == Lk,
+                    "attention_bias: operands");
+  Tensor m = (bias.stride(3) == 1 || Lk == 1 ? bias : bias.contiguous()).expand({B, H, Lq, Lk});
+  Tensor out = empty_bf16({B, Lq, H, D}, q);
+  EriAttnStrides ld = {};
+  ld.q = token_stride(q); ld.k = token_stride(k); ld.v = token_stride(v);
+  TORCH_CHECK_VALUE(ld.q && ld.k && ld.v, "attention_bias: unsupported operand strides");
+  check(L.eri_flash_attn_bias_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), m.data_ptr(), m.stride(0), m.stride(1),
+                                  m.stride(2), is_bool, (int)B, (int)H, (int)Lq, (int)Lk, (int)D, (float)scale, &ld, stream()),
+        "flash_attn_bias");
+  return out;
+}
+
 // Self-attention of a packed projection whose queries and keys are first normalised (RMS over the whole width) and
 // rotated: attention(rope(norm(q) * wq), rope(norm(k) * wk), v). q, k, v are read and their gradients written inside
 // the packed tensors.

@@ -75,6 +75,8 @@ using torch::autograd::variable_list;
   X(eri_rows_wgrad, (const void*, int, const void*, int, void*, int, int, int, int, int, float, void*))          \
   X(eri_rows_dgrad, (const void*, int, const void*, int, float*, int, int, int, int, void*))                     \
   X(eri_gemv_bf16, (const void*, const void*, const void*, void*, int, int, int, int, int, int, int, int, void*)) \
+  X(eri_flash_attn_bias_fwd, (const void*, const void*, const void*, void*, const void*, long long, long long,   \
+                              long long, int, int, int, int, int, int, float, const EriAttnStrides*, void*))     \
   X(eri_flash_attn_wide_fwd, (const void*, const void*, const void*, void*, int, int, int, int, float,           \
                               const EriAttnStrides*, void*))                                                     \
   X(eri_norm_rope_fwd, (const void*, const void*, long long, const void*, const void*, const float*, const float*, \
@@ -187,6 +189,7 @@ Tensor attention(const Tensor& q, const Tensor& k, const Tensor& v, double scale
 Tensor attention_qkv(const Tensor& qkv, int64_t heads, double scale, const OptT& kbias);
 Tensor attention_kv(const Tensor& q, const Tensor& kv, int64_t heads, double scale, const OptT& kbias);
 Tensor attention_wide(const Tensor& q, const Tensor& k, const Tensor& v, double scale);
+Tensor attention_bias(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& bias, double scale);
 Tensor attention_qkv_rope(const Tensor& qkv, const Tensor& wq, const Tensor& wk, const Tensor& cos, const Tensor& sin,
                           int64_t heads, double eps);
 Tensor mse_loss(const Tensor& pred, const Tensor& target, const OptT& weight);

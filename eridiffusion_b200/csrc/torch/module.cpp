@@ -48,6 +48,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attention_qkv", &attention_qkv);
   m.def("attention_kv", &attention_kv);
   m.def("attention_wide", &attention_wide);
+  m.def("attention_bias", &attention_bias);
   m.def("attention_qkv_rope", &attention_qkv_rope);
   m.def("mse_loss", &mse_loss);
   m.def("group_norm_silu", &group_norm_silu);

@@ -65,8 +65,8 @@ class _ClipLayer(nn.Module):
 
     def forward(self, x, mask):
         B, T, D = x.shape
-        q, k, v = self.qkv(self.ln1(x)).view(B, T, 3, self.heads, D // self.heads).unbind(2)
-        x = x + self.out(F.attention(q.contiguous(), k.contiguous(), v.contiguous(), mask=mask).reshape(B, T, D))
+        q, k, v = self.qkv(self.ln1(x)).view(B, T, 3, self.heads, D // self.heads).unbind(2)    # read in place
+        x = x + self.out(F.attention(q, k, v, mask=mask).reshape(B, T, D))
         h = self.fc1(self.ln2(x))
         h = h * torch.sigmoid(1.702 * h) if self.act == "quick_gelu" else TF.gelu(h)
         return x + self.fc2(h)
@@ -144,9 +144,9 @@ class _T5Layer(nn.Module):
         B, T, _ = x.shape
         q, k, v = self.qkv(self.ln1(x)).view(B, T, 3, self.heads, self.head_dim).unbind(2)
         # T5 attention is unscaled and carries an additive relative-position bias
-        o = F.attention(q.contiguous(), k.contiguous(), v.contiguous(), scale=1.0, mask=bias)
-        x = x + self.o(o.reshape(B, T, -1))
-        return x + self.wo(F.glu(self.wi(self.ln2(x)), "gelu", act_first=True))
+        o = F.attention(q, k, v, scale=1.0, mask=bias)
+        x = self.o(o.reshape(B, T, -1), residual=x)
+        return self.wo(F.glu(self.wi(self.ln2(x)), "gelu", act_first=True), residual=x)
 
 
 class T5Encoder(nn.Module):

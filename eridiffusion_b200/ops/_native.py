@@ -180,7 +180,7 @@ def debug_bounds_report() -> dict:
     if h is None:
         return out
     buf = (C.c_int * 4)()
-    for tag in ("gemm", "gemm2", "tokred", "fa", "fa_wide", "route"):
+    for tag in ("gemm", "gemm2", "tokred", "fa", "fa_wide", "fa_bias", "route"):
         fn = getattr(h, f"eri_{tag}_debug_bounds", None)
         if fn is None:
             if DEBUG_BOUNDS:

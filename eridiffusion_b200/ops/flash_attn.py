@@ -29,6 +29,7 @@ N._SIGNATURES.update({
     "eri_fa_check_error": [],
     "eri_fa2_check_error": [],
     "eri_fa_wide_check_error": [],
+    "eri_fa_bias_check_error": [],
     "eri_fa_bwd_check_error": [],
 })
 
@@ -41,7 +42,7 @@ def _bind(lib):
     for name in ("eri_flash_attn_fwd", "eri_flash_attn_bwd", "eri_flash_attn_fwd_ld", "eri_flash_attn_bwd_ld",
                  "eri_flash_attn_fwd_masked",
                  "eri_flash_attn_bwd_masked", "eri_flash_attn_fwd_pair", "eri_fa_check_error",
-                 "eri_fa2_check_error", "eri_fa_wide_check_error", "eri_fa_bwd_check_error"):
+                 "eri_fa2_check_error", "eri_fa_wide_check_error", "eri_fa_bias_check_error", "eri_fa_bwd_check_error"):
         if hasattr(lib, name):
             fn = getattr(lib, name)
             fn.argtypes = N._SIGNATURES[name]
@@ -260,6 +261,8 @@ def check_error() -> int:
         e = lib.eri_fa2_check_error()
     if not e and hasattr(lib, "eri_fa_wide_check_error"):
         e = lib.eri_fa_wide_check_error()
+    if not e and hasattr(lib, "eri_fa_bias_check_error"):
+        e = lib.eri_fa_bias_check_error()
     if not e and hasattr(lib, "eri_fa_bwd_check_error"):
         e = lib.eri_fa_bwd_check_error()
     return e

@@ -622,6 +622,9 @@ def attention(q, k, v, scale=None, mask=None, out=None):
         if mask is None and out is None and _wide_ok(q, k, v):
             ATTENTION_CALLS["native"] += 1
             return N.ops().attention_wide(q, k, v, scale if scale is not None else 1.0 / math.sqrt(512))
+        if mask is not None and out is None and _bias_ok(q, k, v, mask):
+            ATTENTION_CALLS["native"] += 1
+            return N.ops().attention_bias(q, k, v, mask, scale if scale is not None else 1.0 / math.sqrt(q.shape[-1]))
         # other head sizes below 128 (SD1.5: 40 and 80) ride on the 64 / 128 kernels with zero columns
         # appended: zero query / key columns leave the scores unchanged, zero value columns give zero
         # output columns that are cut off again (the pad and the slice are differentiable copies)
@@ -647,6 +650,15 @@ def _wide_ok(q, k, v) -> bool:
     """Head size 512 (the image autoencoders' middle block), forward only: tiles of 128 queries and 128 keys."""
     return (q.shape[-1] == 512 and q.shape[1] >= 128 and k.shape[1] >= 128 and k.shape == v.shape and q.shape[0] == k.shape[0]
             and q.shape[2] == k.shape[2] and not (torch.is_grad_enabled() and any(t.requires_grad for t in (q, k, v))))
+
+
+def _bias_ok(q, k, v, mask) -> bool:
+    """A mask per query and key (relative-position bias, causal), forward only: bf16 or boolean, a value for every key."""
+    B, Lq, H, D = q.shape
+    return (D in (64, 128) and k.shape == v.shape == (B, k.shape[1], H, D) and mask.device == q.device
+            and mask.dtype in (torch.bool, torch.bfloat16) and mask.dim() == 4 and mask.shape[3] == k.shape[1]
+            and mask.shape[0] in (1, B) and mask.shape[1] in (1, H) and mask.shape[2] in (1, Lq)
+            and not (torch.is_grad_enabled() and any(t.requires_grad for t in (q, k, v, mask))))
 
 
 def _packed_ok(head_dim, mask, B, Lk, *ts) -> bool:
