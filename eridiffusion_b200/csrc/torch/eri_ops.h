@@ -63,6 +63,7 @@ using torch::autograd::variable_list;
   X(eri_gemm_tokred, (const void*, long long, const void*, long long, void*, int, int, int, int, float, int,     \
                       int, long long, void*))                                                                    \
   X(eri_gemm_bf16, (const EriGemmArgs*, void*))                                                                  \
+  X(eri_gemm_few_bf16, (const EriGemmArgs*, void*))                                                              \
   X(eri_gemm2_bf16, (const EriGemmArgs*, void*))                                                                 \
   X(eri_gemm2_bf16_group2, (const EriGemmArgs*, const EriGemmArgs*, void*))                                      \
   X(eri_batched_transpose, (const void*, int, int, void*))                                                       \

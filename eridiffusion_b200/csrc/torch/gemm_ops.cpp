@@ -61,6 +61,11 @@ Built build(const Tensor& a, const Tensor& b, const GemmOpt& o) {
 
 // The choice of kernel, as in ops/functional.py: _launch_gemm.
 void launch(const EriGemmArgs& g, int flags) {
+  // Few 128 x 128 tiles: the K range over a cluster, two CTAs per SM (answers -30 for any other product).
+  if (!g.a_mn || (g.M >= 256 && g.N >= 256)) {
+    const int code = L.eri_gemm_few_bf16(&g, stream());
+    if (code != -30) return check(code, "gemm_few_bf16");
+  }
   // Few pair tiles (the 512-token text stream against a 3072-wide weight: 24 tiles for 74 CTA pairs) leave
   // most SMs idle; the one-CTA kernel's 128-column tiles spread the same work over four times as many CTAs.
   const bool few = !(g.a_mn || g.glu) &&

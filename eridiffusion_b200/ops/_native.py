@@ -117,6 +117,8 @@ _SIGNATURES = {
     "eri_gemm_check_error": [],
     "eri_gemm_bf16": [C.POINTER(GemmArgs), _P],
     "eri_gemm2_bf16": [C.POINTER(GemmArgs), _P],
+    "eri_gemm_few_bf16": [C.POINTER(GemmArgs), _P],
+    "eri_gemm_few_check_error": [],
     "eri_gemm2_bf16_group2": [C.POINTER(GemmArgs), C.POINTER(GemmArgs), _P],
     "eri_gemm2_check_error": [],
     "eri_gemm2_gather_count": [],
@@ -180,7 +182,7 @@ def debug_bounds_report() -> dict:
     if h is None:
         return out
     buf = (C.c_int * 4)()
-    for tag in ("gemm", "gemm2", "tokred", "fa", "fa_wide", "fa_bias", "route"):
+    for tag in ("gemm", "gemm2", "gemm_few", "tokred", "fa", "fa_wide", "fa_bias", "route"):
         fn = getattr(h, f"eri_{tag}_debug_bounds", None)
         if fn is None:
             if DEBUG_BOUNDS:

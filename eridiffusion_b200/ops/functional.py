@@ -268,6 +268,12 @@ def gemm_native(a, b, *, out=None, alpha=1.0, bias=None, lora_h=None, lora_b=Non
 
 def _launch_gemm(lib, g, out, route):
     M, Nn, K, a_mn, glu, gather, scatter, force_bn = route
+    # Few 128 x 128 tiles: the K range over a cluster, two CTAs per SM (answers -30 for any other product).
+    if gather is None and scatter is None and force_bn <= 0 and (not a_mn or (M >= 256 and Nn >= 256)):
+        code = lib.eri_gemm_few_bf16(g, N.stream_ptr())
+        if code != -30:
+            N.check(code, "gemm_few_bf16")
+            return out
     # Few pair tiles (the 512-token text stream against a 3072-wide weight: 24 tiles for 74 CTA pairs)
     # leave most SMs idle; the one-CTA kernel's 128-column tiles spread the same work over four times
     # as many CTAs (measured 22.5 against 30.7 us at 512 x 3072 x 3072, 61 against 78 us at K = 12288).
@@ -380,6 +386,8 @@ def gemm_error_check() -> int:
     e = lib.eri_gemm_check_error()
     if not e and hasattr(lib, "eri_gemm2_check_error"):
         e = lib.eri_gemm2_check_error()
+    if not e and hasattr(lib, "eri_gemm_few_check_error"):
+        e = lib.eri_gemm_few_check_error()
     return e
 
 
