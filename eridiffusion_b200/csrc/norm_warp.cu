@@ -418,8 +418,174 @@ __global__ void __launch_bounds__(1024, 1) norm_rows_smem_kernel(const NormArgs 
   }
 }
 
+// ---- one row per CTA of 128 threads, in registers ----
+// For few rows. The row-per-warp kernel above wants rows for every warp of an SM: 256 rows x 4096 ran on 10 SMs, and a
+// row was a chain of a bulk copy and two walks of 16 dependent shared-memory reads (13 us). Here every SM has rows,
+// the row's loads and the modulation's are all in flight at once, and the sums are exact two-pass ones.
+constexpr int kRowThreads = 128;
+
+__device__ __forceinline__ float2 row_sum2(float a, float b, float2* sm) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+  }
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = make_float2(a, b);
+  __syncthreads();
+  float2 t = sm[0];
+#pragma unroll
+  for (int i = 1; i < kRowThreads / 32; ++i) {
+    t.x += sm[i].x;
+    t.y += sm[i].y;
+  }
+  return t;
+}
+
+// V: 16-byte vectors per thread (D <= 8 * V * 128)
+template <bool BWD, int V>
+__global__ void __launch_bounds__(kRowThreads) norm_row_cta_kernel(const NormArgs a) {
+  __shared__ float2 sm[2][kRowThreads / 32];
+  const int row = blockIdx.x, D = a.D, nvec = D >> 3;
+  const size_t mod = (size_t)(row / a.rows_per_batch) * a.mod_stride;
+  const float inv_d = 1.f / (float)D;
+  bf16x8 x[V], g[V], sc[V], ex[V], wv[V], bv[V];   // ex: shift (forward) or addend (backward)
+#pragma unroll
+  for (int u = 0; u < V; ++u) {
+    const int v = threadIdx.x + u * kRowThreads;
+    if (v >= nvec) continue;
+    x[u] = reinterpret_cast<const bf16x8*>(a.x + (size_t)row * D)[v];
+    if (BWD) g[u] = reinterpret_cast<const bf16x8*>(a.dy + (size_t)row * D)[v];
+    if (a.scale) sc[u] = reinterpret_cast<const bf16x8*>(a.scale + mod)[v];
+    if (a.weight) wv[u] = reinterpret_cast<const bf16x8*>(a.weight)[v];
+    if (!BWD) {
+      if (a.shift) ex[u] = reinterpret_cast<const bf16x8*>(a.shift + mod)[v];
+      if (a.bias) bv[u] = reinterpret_cast<const bf16x8*>(a.bias)[v];
+    } else if (a.addend) {
+      ex[u] = reinterpret_cast<const bf16x8*>(a.addend + (size_t)row * D)[v];
+    }
+  }
+  bf16x8* out = reinterpret_cast<bf16x8*>(a.out + (size_t)row * D);
+  if constexpr (!BWD) {
+    float mean = 0.f;
+    if (!a.rms) {
+      float s = 0.f;
+#pragma unroll
+      for (int u = 0; u < V; ++u)
+        if (threadIdx.x + u * kRowThreads < nvec) {
+          float f[8];
+          unpack8(x[u], f);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) s += f[j];
+        }
+      mean = row_sum2(s, 0.f, sm[0]).x * inv_d;
+    }
+    float q = 0.f;
+#pragma unroll
+    for (int u = 0; u < V; ++u)
+      if (threadIdx.x + u * kRowThreads < nvec) {
+        float f[8];
+        unpack8(x[u], f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) q = fmaf(f[j] - mean, f[j] - mean, q);
+      }
+    const float rstd = rsqrtf(row_sum2(q, 0.f, sm[1]).x * inv_d + a.eps);
+    if (threadIdx.x == 0) {
+      if (a.mean) a.mean[row] = mean;
+      if (a.rstd) a.rstd[row] = rstd;
+    }
+#pragma unroll
+    for (int u = 0; u < V; ++u) {
+      const int v = threadIdx.x + u * kRowThreads;
+      if (v >= nvec) continue;
+      float f[8], t[8];
+      unpack8(x[u], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = (f[j] - mean) * rstd;
+      if (a.weight) {
+        unpack8(wv[u], t);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] *= t[j];
+      }
+      if (a.bias) {
+        unpack8(bv[u], t);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] += t[j];
+      }
+      if (a.scale) {
+        unpack8(sc[u], t);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = fmaf(f[j], t[j], f[j]);
+      }
+      if (a.shift) {
+        unpack8(ex[u], t);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] += t[j];
+      }
+      out[v] = pack8(f);
+    }
+  } else {
+    const float mean = a.rms ? 0.f : a.mean[row], rstd = a.rstd[row];
+    // g = dy * (1 + scale) * weight
+    auto grad8 = [&](int u, float (&f)[8]) {
+      float t[8];
+      unpack8(g[u], f);
+      if (a.scale) {
+        unpack8(sc[u], t);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = fmaf(f[j], t[j], f[j]);
+      }
+      if (a.weight) {
+        unpack8(wv[u], t);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] *= t[j];
+      }
+    };
+    float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int u = 0; u < V; ++u)
+      if (threadIdx.x + u * kRowThreads < nvec) {
+        float f[8], gg[8];
+        unpack8(x[u], f);
+        grad8(u, gg);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          s1 += gg[j];
+          s2 = fmaf(gg[j], f[j] - mean, s2);
+        }
+      }
+    const float2 s = row_sum2(s1, s2, sm[0]);
+    const float c1 = a.rms ? 0.f : s.x * inv_d, c2 = s.y * inv_d * rstd;      // mean(g), mean(g * xhat)
+#pragma unroll
+    for (int u = 0; u < V; ++u) {
+      const int v = threadIdx.x + u * kRowThreads;
+      if (v >= nvec) continue;
+      float f[8], gg[8];
+      unpack8(x[u], f);
+      grad8(u, gg);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = rstd * (gg[j] - c1 - (f[j] - mean) * rstd * c2);
+      if (a.addend) {
+        unpack8(ex[u], gg);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] += gg[j];
+      }
+      out[v] = pack8(f);
+    }
+  }
+}
+
 int* g_norm_err = nullptr;
 int g_norm_sms = 0;
+
+template <bool BWD>
+int launch_row_cta(const NormArgs& a, cudaStream_t st) {
+  if (a.D <= 1024) norm_row_cta_kernel<BWD, 1><<<a.rows, kRowThreads, 0, st>>>(a);
+  else if (a.D <= 2048) norm_row_cta_kernel<BWD, 2><<<a.rows, kRowThreads, 0, st>>>(a);
+  else if (a.D <= 3072) norm_row_cta_kernel<BWD, 3><<<a.rows, kRowThreads, 0, st>>>(a);
+  else norm_row_cta_kernel<BWD, 4><<<a.rows, kRowThreads, 0, st>>>(a);
+  return (int)cudaGetLastError();
+}
+int g_row_cta_rows = -1;   // tuning hook, see eri_norm_set_row_cta_rows
 
 // ERI_B200_NORM_SMEM=0 (or eri_norm_set_smem_variant(0)) keeps the register-resident kernel.
 int g_norm_smem = -1;
@@ -452,10 +618,20 @@ int launch_rows_smem(const NormArgs& a, cudaStream_t st) {
   return (int)cudaGetLastError();
 }
 
+// A CTA per row up to this many rows, and in the backward wherever a row pair is wide: the row-per-warp kernel then holds
+// fewer than 27 rows per SM. us, row per warp / CTA per row (rows x width):
+//   forward   256x4096 12.1 / 3.1, 1024x1280 6.5 / 3.5, 1536x3072 11.6 / 6.7, 2560x3072 12.2 / 9.4; 4096x1280 7.3 / 8.7,
+//             4608x3072 13.7 / 14.5, 19008x4096 62 / 75
+//   backward  256x4096 11.1 / 3.1, 1024x1280 7.7 / 3.4, 2560x3072 20.2 / 10.8, 9216x3072 47.8 / 35.1, 19008x4096 121 / 91;
+//             4096x640 6.1 / 6.3, 8192x1280 15.1 / 15.7, 16384x640 17.5 / 18.8
+constexpr int kRowCtaRows = 3072, kRowCtaWidth = 2048;
+
 template <bool BWD>
 int launch_rows(const NormArgs& a, cudaStream_t st) {
   constexpr int NT = BWD ? 2 : 1;
   const int D = a.D;
+  const bool row_cta = g_row_cta_rows >= 0 ? a.rows <= g_row_cta_rows : a.rows <= kRowCtaRows || (BWD && D > kRowCtaWidth);
+  if (a.rows > 0 && row_cta) return launch_row_cta<BWD>(a, st);
   if (norm_smem_variant()) {
     const int code = launch_rows_smem<BWD>(a, st);
     if (code != -100) return code;
@@ -508,6 +684,12 @@ int eri_norm_set_smem_variant(int on) {
   const int prev = norm_smem_variant() ? 1 : 0;
   g_norm_smem = on ? 1 : 0;
   return prev;
+}
+
+// Tuning hook: the most rows that take the CTA-per-row kernel (negative: the default rule).
+int eri_norm_set_row_cta_rows(int rows) {
+  g_row_cta_rows = rows;
+  return 0;
 }
 
 // 0, or 1 when a bounded wait for a row copy ran out (the word is cleared by the read).
