@@ -177,7 +177,7 @@ class T5Encoder(nn.Module):
         bias = self.rel_bias(self._buckets(T, ids.device)).permute(2, 0, 1)[None].to(x.dtype)   # [1, H, T, T]
         if key_mask is not None:
             bias = bias + (~key_mask)[:, None, None, :].to(x.dtype) * -1e4
-        bias = bias.expand(B, -1, -1, -1)
+        bias = bias.contiguous().expand(B, -1, -1, -1)      # keys consecutive: the layers read it as it is
         for ly in self.layers:
             x = ly(x, bias)
         return self.final_ln(x)
