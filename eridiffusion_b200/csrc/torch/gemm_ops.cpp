@@ -4,6 +4,9 @@
 // programmatic dependent.
 #include "eri_ops.h"
 
+#include <torch/csrc/autograd/graph_task.h>
+#include <torch/csrc/autograd/variable.h>
+
 #include <mutex>
 #include <unordered_map>
 
@@ -90,7 +93,11 @@ Tensor undef() { return Tensor(); }
 bool gemm_supported(int64_t M, int64_t N, int64_t K) { return M >= 128 && N >= 16 && K >= 8 && K % 8 == 0 && N % 8 == 0; }
 bool lora_rank_ok(int64_t r) { return r == 16 || r == 32 || r == 64; }
 bool has_grad_buffer(const Tensor& p, at::ScalarType t) {
-  if (!p.is_leaf()) return false;
+  if (!p.is_leaf() || !p.requires_grad()) return false;
+  // torch.autograd.grad and backward(inputs=...) want the gradient itself, and so does whoever hooked the parameter
+  const auto* asked = torch::autograd::get_current_graph_task_exec_info();
+  if (asked && !asked->empty()) return false;
+  if (!torch::autograd::impl::hooks(p).empty() || torch::autograd::impl::post_acc_grad_hooks(p)) return false;
   const Tensor& g = p.grad();
   return g.defined() && g.scalar_type() == t && g.is_contiguous();
 }
