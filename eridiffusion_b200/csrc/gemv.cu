@@ -108,20 +108,21 @@ extern "C" int eri_gemv_bf16(const void* x, const void* w, const void* bias, voi
 // (crates/training/src/flux/runtime.rs:401-463 forward; gradients through the autograd tape).
 namespace {
 
+// T rows; ACC: added to what dW holds. A CTA owns 128 x 8 columns of dW and walks its rows in chunks of kChunk whose dy
+// values are staged in shared memory. The old values of four rows are loaded before any of them is written: a load may
+// not pass an earlier store to the same tensor, and one row in flight per thread reached 3.3 TB/s (68 us for an
+// 18432 x 3072 gradient, 226 MB).
+template <int T, bool ACC>
 __global__ void __launch_bounds__(128) rows_wgrad_kernel(const bf16* __restrict__ dy, int ldy, const bf16* __restrict__ x,
-                                                         int ldx, bf16* __restrict__ dw, int ldw, int T, int N, int K,
-                                                         int accumulate, float scale) {
-  // a CTA owns 128 x 8 columns of dW and walks its rows in chunks of kChunk: the chunk's dy values are
-  // staged in shared memory first, so that the row loop has no dependent global load in it
-  constexpr int kChunk = 64;
-  __shared__ float sdy[kMaxM][kChunk];
+                                                         int ldx, bf16* __restrict__ dw, int ldw, int N, int K, float scale) {
+  constexpr int kChunk = 64, kRows = 4;
+  __shared__ float sdy[T][kChunk];
   const int kv = blockIdx.x * blockDim.x + threadIdx.x;   // 8 columns per thread
   const bool live = kv * 8 < K;
-  float xf[kMaxM][8];
+  float xf[T][8];
 #pragma unroll
-  for (int t = 0; t < kMaxM; ++t) {
-    if (t < T && live) unpack8(*reinterpret_cast<const bf16x8*>(x + (size_t)t * ldx + kv * 8), xf[t]);
-  }
+  for (int t = 0; t < T; ++t)
+    if (live) unpack8(*reinterpret_cast<const bf16x8*>(x + (size_t)t * ldx + kv * 8), xf[t]);
   for (int n0 = blockIdx.y * kChunk; n0 < N; n0 += gridDim.y * kChunk) {
     const int nc = min(kChunk, N - n0);
     __syncthreads();
@@ -131,25 +132,32 @@ __global__ void __launch_bounds__(128) rows_wgrad_kernel(const bf16* __restrict_
     }
     __syncthreads();
     if (!live) continue;
-#pragma unroll 4
-    for (int j = 0; j < nc; ++j) {
-      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    bf16* o = dw + (size_t)n0 * ldw + kv * 8;
+    for (int j0 = 0; j0 < nc; j0 += kRows) {
+      bf16x8 old[kRows];
+      if (ACC) {
 #pragma unroll
-      for (int t = 0; t < kMaxM; ++t) {
-        if (t < T) {
-          const float d = sdy[t][j];
+        for (int u = 0; u < kRows; ++u)
+          if (j0 + u < nc) old[u] = *reinterpret_cast<const bf16x8*>(o + (size_t)(j0 + u) * ldw);
+      }
+#pragma unroll
+      for (int u = 0; u < kRows; ++u) {
+        if (j0 + u >= nc) break;
+        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+          const float d = sdy[t][j0 + u];
 #pragma unroll
           for (int q = 0; q < 8; ++q) acc[q] = fmaf(d, xf[t][q], acc[q]);
         }
-      }
-      bf16x8* o = reinterpret_cast<bf16x8*>(dw + (size_t)(n0 + j) * ldw + kv * 8);
-      if (accumulate) {
-        float old[8];
-        unpack8(*o, old);
+        if (ACC) {
+          float w[8];
+          unpack8(old[u], w);
 #pragma unroll
-        for (int q = 0; q < 8; ++q) acc[q] += old[q];
+          for (int q = 0; q < 8; ++q) acc[q] += w[q];
+        }
+        *reinterpret_cast<bf16x8*>(o + (size_t)(j0 + u) * ldw) = pack8(acc);
       }
-      *o = pack8(acc);
     }
   }
 }
@@ -200,8 +208,20 @@ extern "C" int eri_rows_wgrad(const void* dy, int ldy, const void* x, int ldx, v
   if (gy > chunks) gy = chunks;
   if (gy > 65535) gy = 65535;
   dim3 grid(gx, gy);
-  rows_wgrad_kernel<<<grid, block, 0, (cudaStream_t)stream>>>((const bf16*)dy, ldy, (const bf16*)x, ldx,
-                                                              (bf16*)dw, ldw, T, N, K, accumulate, scale);
+#define ERI_WGRAD_CASE(TT)                                                                                      \
+  case TT:                                                                                                      \
+    if (accumulate)                                                                                             \
+      rows_wgrad_kernel<TT, true><<<grid, block, 0, (cudaStream_t)stream>>>((const bf16*)dy, ldy, (const bf16*)x, ldx, \
+                                                                            (bf16*)dw, ldw, N, K, scale);       \
+    else                                                                                                        \
+      rows_wgrad_kernel<TT, false><<<grid, block, 0, (cudaStream_t)stream>>>((const bf16*)dy, ldy, (const bf16*)x, ldx, \
+                                                                             (bf16*)dw, ldw, N, K, scale);      \
+    break;
+  switch (T) {
+    ERI_WGRAD_CASE(1) ERI_WGRAD_CASE(2) ERI_WGRAD_CASE(3) ERI_WGRAD_CASE(4)
+    ERI_WGRAD_CASE(5) ERI_WGRAD_CASE(6) ERI_WGRAD_CASE(7) ERI_WGRAD_CASE(8)
+  }
+#undef ERI_WGRAD_CASE
   return (int)cudaGetLastError();
 }
 
