@@ -225,6 +225,7 @@ class UnifiedInferencePipeline:
         p = next(model.parameters())
         self.device = torch.device(device) if device is not None else p.device
         self.dtype = dtype or p.dtype
+        self._train_sigmas = {}          # device -> the training chain's noise levels
         self.memory = memory or model_type.memory_config(
             torch.cuda.get_device_properties(self.device).total_memory / 2 ** 30 if self.device.type == "cuda" else 180.0)
         if self.memory.cpu_offload:
@@ -280,8 +281,11 @@ class UnifiedInferencePipeline:
     def _generate_sdxl(self, ctx, pooled, neg_ctx, neg_pooled, width, height, steps, scale, seed, sampler):
         m, dev, dt = self.model, self.device, self.dtype
         B = ctx.shape[0]
-        tid = torch.tensor([[height, width, 0, 0, height, width]] * B, dtype=torch.float32, device=dev)
-        train_sigmas = ddpm_sigmas().to(dev)
+        # made on the device: a copy from pageable host memory would wait for the image before this one
+        tid = torch.stack([torch.full((B,), float(v), device=dev) for v in (height, width, 0, 0, height, width)], 1)
+        train_sigmas = self._train_sigmas.get(dev)
+        if train_sigmas is None:
+            train_sigmas = self._train_sigmas[dev] = ddpm_sigmas().to(dev)
         eps = lambda x, t: m(x, t, ctx, pooled, tid)
         den = eps_denoiser(eps, train_sigmas)
         if scale != 1.0:
