@@ -796,6 +796,47 @@ Tensor upsample2x(const Tensor& x) {
   return Upsample2x::run(rows_contig(x), false);
 }
 
+// Convolution (no bias, one group) with a trained weight in the parameter order [Co, Ci, kh, kw]: the channels-last copy that
+// the library reads is made once for both directions, and the weight gradient is added into the parameter's gradient
+// in the pass that brings it back into that order.
+namespace {
+struct TrainedConv : torch::autograd::Function<TrainedConv> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, std::vector<int64_t> strides,
+                        std::vector<int64_t> padding, std::vector<int64_t> dilation) {
+    Tensor rows = at::empty(w.sizes(), w.options(), at::MemoryFormat::ChannelsLast);
+    check(L.eri_conv_weight_order(w.data_ptr(), rows.data_ptr(), (int)w.size(0), (int)w.size(1), (int)(w.size(2) * w.size(3)), 0,
+                                  stream()), "conv_weight_order");
+    ctx->save_for_backward({x, w, rows});
+    ctx->saved_data["s"] = strides;
+    ctx->saved_data["p"] = padding;
+    ctx->saved_data["d"] = dilation;
+    return at::conv2d(x, rows, {}, strides, padding, dilation, 1);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    auto sv = ctx->get_saved_variables();
+    const Tensor &x = sv[0], &w = sv[1], &rows = sv[2];
+    const bool nx = ctx->needs_input_grad(0), nw = ctx->needs_input_grad(1);
+    auto [dx, dw, db] = at::convolution_backward(g[0], x, rows, std::nullopt, ctx->saved_data["s"].toIntVector(),
+                                                 ctx->saved_data["p"].toIntVector(), ctx->saved_data["d"].toIntVector(), false,
+                                                 std::vector<int64_t>{0, 0}, 1, {nx, nw, false});
+    if (nw && has_grad_buffer(w, at::kBFloat16) && al16(w.grad())) {
+      Tensor d = dw.contiguous(at::MemoryFormat::ChannelsLast);
+      if (al16(d)) {
+        check(L.eri_conv_weight_order(d.data_ptr(), w.grad().data_ptr(), (int)w.size(0), (int)w.size(1),
+                                      (int)(w.size(2) * w.size(3)), 1, stream()), "conv_weight_order");
+        dw = Tensor();
+      }
+    }
+    return {dx, dw, Tensor(), Tensor(), Tensor()};
+  }
+};
+}  // namespace
+
+Tensor conv2d_trained(const Tensor& x, const Tensor& w, const std::vector<int64_t>& strides, const std::vector<int64_t>& padding,
+                      const std::vector<int64_t>& dilation) {
+  return TrainedConv::apply(x, w, strides, padding, dilation);
+}
+
 // ------------------------------------------------------------------------------- FLUX single-stream block
 // x + gate * linear2(cat(attn(qkv), gelu(mlp))) where qkv and mlp are column ranges of one projection linear1. The
 // column-split epilogue of the GEMM writes both straight to where the next op reads them, and backward produces

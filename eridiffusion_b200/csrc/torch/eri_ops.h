@@ -54,6 +54,7 @@ using torch::autograd::variable_list;
   X(eri_gn_bwd, (const void*, const void*, const void*, const void*, const void*, const void*, const float*,     \
                  const float*, void*, void*, void*, void*, void*, float*, int, int, int, int, int, int, void*))  \
   X(eri_add_bias, (const void*, const void*, const void*, const void*, void*, long long, int, void*))            \
+  X(eri_conv_weight_order, (const void*, void*, int, int, int, int, void*))                                      \
   X(eri_upsample2x, (const void*, void*, long long, int, int, int, void*))                                       \
   X(eri_gemm_skinny, (const void*, long long, const void*, long long, void*, int, int, int, int, float, void*))  \
   X(eri_gemm_rank_stream, (const void*, long long, const void*, long long, void*, int, int, int, int, float,     \
@@ -198,6 +199,8 @@ Tensor group_norm_silu(const Tensor& x, const Tensor& weight, const OptT& bias, 
                        int64_t groups, double eps, bool silu);
 Tensor add_bias(const Tensor& a, const Tensor& b, const OptT& bias, const OptT& bias2);
 Tensor upsample2x(const Tensor& x);
+Tensor conv2d_trained(const Tensor& x, const Tensor& w, const std::vector<int64_t>& stride, const std::vector<int64_t>& padding,
+                      const std::vector<int64_t>& dilation);
 Tensor single_stream(const Tensor& xm, const Tensor& x, const Tensor& gate, const Tensor& w1, const OptT& b1,
                      const Tensor& w2, const OptT& b2, const OptT& a1, const OptT& bb1, double s1, const OptT& a2,
                      const OptT& bb2, double s2, const OptT& qs, const OptT& ks, const OptT& cos, const OptT& sin,

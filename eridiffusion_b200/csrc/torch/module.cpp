@@ -53,6 +53,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("mse_loss", &mse_loss);
   m.def("group_norm_silu", &group_norm_silu);
   m.def("add_bias", &add_bias);
+  m.def("conv2d_trained", &conv2d_trained);
   m.def("upsample2x", &upsample2x);
   m.def("single_stream", &single_stream);
 }

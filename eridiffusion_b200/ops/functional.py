@@ -841,6 +841,11 @@ def conv_no_bias(conv, x):
         Nn, C, H, W = x.shape
         rows = x.permute(0, 2, 3, 1).reshape(Nn, H * W, C)
         return linear(rows, w.view(w.shape[0], C)).view(Nn, H, W, w.shape[0]).permute(0, 3, 1, 2)
+    if torch.is_grad_enabled() and w.requires_grad and _native_ok(x, w) and conv.groups == 1 and not isinstance(conv.padding, str) \
+            and w.is_contiguous() and w.shape[1] % 8 == 0 and w.shape[0] <= 65535 and 1 < w.shape[2] * w.shape[3] <= 25 \
+            and w.data_ptr() % 16 == 0:
+        # (a parameter of the flat arena; a weight already in channels-last order needs no copy)
+        return N.ops().conv2d_trained(x, w, list(conv.stride), list(conv.padding), list(conv.dilation))
     return torch.nn.functional.conv2d(x, w, None, conv.stride, conv.padding, conv.dilation, conv.groups)
 
 
