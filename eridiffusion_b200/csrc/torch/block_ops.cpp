@@ -418,6 +418,9 @@ std::pair<Tensor, Tensor> attn_fwd(const Tensor& q, const Tensor& k, const Tenso
   EriAttnStrides ld = {};
   ld.q = token_stride(q); ld.k = token_stride(k); ld.v = token_stride(v); ld.out = token_stride(out);
   TORCH_CHECK_VALUE(ld.q && ld.k && ld.v && ld.out, "flash attention: unsupported operand strides");
+  // the kernels walk the keys with q's batch, head count and head size
+  TORCH_CHECK_VALUE(k.size(0) == B && k.size(2) == H && k.size(3) == D && v.sizes() == k.sizes(), "flash attention: q ", q.sizes(),
+                    " does not go with k ", k.sizes(), " and v ", v.sizes());
   Tensor lse = empty_f32({B, H, Lq}, q);
   if (pair_poly >= 0 && !kbias.defined() && out.is_contiguous() && q.is_contiguous() && k.is_contiguous() &&
       v.is_contiguous() && D == 128 && Lq >= 256 && Lk >= 128) {

@@ -671,7 +671,7 @@ def _bias_ok(q, k, v, mask) -> bool:
 
 def _packed_ok(head_dim, mask, B, Lk, *ts) -> bool:
     from . import flash_attn as FA
-    return (_ATTN_NATIVE == "native" and head_dim in (64, 128) and _native_ok(*ts) and ts[0].shape[1] >= 16 and FA.has_forward()
+    return (_ATTN_NATIVE == "native" and head_dim in (64, 128) and _native_ok(*ts) and ts[0].shape[1] >= 16 and Lk >= 1 and FA.has_forward()
             and (mask is None or FA.mask_is_key_only(mask, B, Lk)))
 
 
@@ -693,7 +693,7 @@ def attention_kv(q, kv, num_heads, scale=None, mask=None):
     """Cross-attention of q [B, L, H*Dh] on a packed key / value projection [B, Lk, 2*H*Dh] -> [B, L, H*Dh]."""
     B, L, W = q.shape
     Lk, Dh = kv.shape[1], W // num_heads
-    if _packed_ok(Dh, mask, B, Lk, q, kv):
+    if kv.shape[0] == B and kv.shape[2] == 2 * W and _packed_ok(Dh, mask, B, Lk, q, kv):
         from . import flash_attn as FA
         ATTENTION_CALLS["native"] += 1
         kb = None if mask is None else FA.key_bias(mask, B, Lk, q.device)
