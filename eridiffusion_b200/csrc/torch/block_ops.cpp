@@ -680,6 +680,11 @@ Tensor rows_contig(const Tensor& x) {
   return al16(c) ? c : c.clone();      // (a clone keeps the memory format)
 }
 
+// The kernels index these by channel (and sample): a shorter tensor would be read past its end.
+void check_channels(const Tensor& t, int64_t n, const char* what) {
+  TORCH_CHECK_VALUE(!t.defined() || t.numel() == n, what, ": ", t.sizes(), " where ", n, " values are needed");
+}
+
 // GroupNorm (+SiLU) of x + pre_c + pre_nc: the bias of the convolution before it and a per-sample embedding are added
 // where x is read.
 Tensor gn_forward(const Tensor& x, const Tensor& w, const Tensor& b, const Tensor& pc, const Tensor& pn, int64_t groups,
@@ -781,6 +786,13 @@ struct Upsample2x : torch::autograd::Function<Upsample2x> {
 Tensor group_norm_silu(const Tensor& x, const Tensor& w, const OptT& b_, const OptT& pc_, const OptT& pn_, int64_t groups,
                        double eps, bool silu) {
   Tensor b = opt(b_), pc = opt(pc_), pn = opt(pn_);
+  const Rows r(x);
+  check_channels(w, r.C, "group_norm_silu weight");
+  check_channels(b, r.C, "group_norm_silu bias");
+  check_channels(pc, r.C, "group_norm_silu pre_c");
+  if (pn.defined() && pn.dim() == 2 && pn.size(0) == 1 && r.N != 1) pn = pn.expand({r.N, pn.size(1)});   // one embedding for all samples
+  check_channels(pn, (int64_t)r.N * r.C, "group_norm_silu pre_nc");
+  TORCH_CHECK_VALUE(!pn.defined() || (pn.dim() == 2 && pn.size(0) == r.N), "group_norm_silu pre_nc: ", pn.sizes());
   if (any_grad({&x, &w, &b, &pc, &pn}))
     return GroupNormSilu::apply(wrap(x), wrap(w), wrap(b), wrap(pc), wrap(pn), groups, eps, silu);
   return gn_forward(rows_contig(x), contig16(w), contig16(b), contig16(pc), contig16(pn), groups, eps, silu, Tensor());
@@ -789,6 +801,10 @@ Tensor group_norm_silu(const Tensor& x, const Tensor& w, const OptT& b_, const O
 // a + b + bias + bias2 (per channel): a block's residual sum with the biases of its last convolutions.
 Tensor add_bias(const Tensor& a, const Tensor& b, const OptT& bias_, const OptT& bias2_) {
   Tensor bias = opt(bias_), bias2 = opt(bias2_);
+  const Rows r(a);
+  TORCH_CHECK_VALUE(a.sizes() == b.sizes(), "add_bias: ", a.sizes(), " and ", b.sizes());
+  check_channels(bias, r.C, "add_bias bias");
+  check_channels(bias2, r.C, "add_bias bias2");
   if (any_grad({&a, &b, &bias, &bias2})) return AddBias::apply(wrap(a), wrap(b), wrap(bias), wrap(bias2));
   return add_bias_forward(rows_contig(a), rows_contig(b), contig16(bias), contig16(bias2));
 }
