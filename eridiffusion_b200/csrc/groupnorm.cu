@@ -418,6 +418,7 @@ extern "C" {
 
 // fp32 words of workspace one call needs.
 long long eri_gn_workspace(int N, int HW, int C, int G, int backward) {
+  if (N < 1 || HW < 1 || C < 8) return 0;      // nothing to plan (the calls below refuse it)
   const GnPlan p = plan_for(N, HW, C);
   return (long long)N * (p.chunks + 1) * G * 2 + (backward ? (long long)N * p.chunks * C * 3 : 0);
 }
@@ -426,7 +427,7 @@ long long eri_gn_workspace(int N, int HW, int C, int G, int backward) {
 // pre_nc [N, C] (bf16) may be null.
 int eri_gn_fwd(const void* x, const void* pre_c, const void* pre_nc, const void* w, const void* b, void* y, float* mean,
                float* rstd, float* ws, int N, int HW, int C, int G, float eps, int silu, void* stream) {
-  if (C % 8 || C % G) return -1;
+  if (N < 1 || HW < 1 || C < 8 || G < 1 || C % 8 || C % G) return -1;
   GnArgs a = {};
   a.x = (const bf16*)x; a.w = (const bf16*)w; a.b = (const bf16*)b; a.out = (bf16*)y; a.mean = mean; a.rstd = rstd;
   a.pre_c = (const bf16*)pre_c; a.pre_nc = (const bf16*)pre_nc;
@@ -439,7 +440,7 @@ int eri_gn_fwd(const void* x, const void* pre_c, const void* pre_nc, const void*
 int eri_gn_bwd(const void* x, const void* pre_c, const void* pre_nc, const void* dy, const void* w, const void* b,
                const float* mean, const float* rstd, void* dx, void* dw, void* db, void* dpre_c, void* dpre_nc, float* ws,
                int N, int HW, int C, int G, int silu, int accumulate, void* stream) {
-  if (C % 8 || C % G) return -1;
+  if (N < 1 || HW < 1 || C < 8 || G < 1 || C % 8 || C % G) return -1;
   GnArgs a = {};
   a.x = (const bf16*)x; a.dy = (const bf16*)dy; a.w = (const bf16*)w; a.b = (const bf16*)b;
   a.pre_c = (const bf16*)pre_c; a.pre_nc = (const bf16*)pre_nc;

@@ -62,3 +62,10 @@ def test_one_embedding_for_every_sample():
     want = wide.grad.double().sum(0, keepdim=True)
     # three bf16 values added and rounded once: 2^-8 of the largest partial sum
     assert (emb.grad.double() - want).abs().max() <= 2.0 ** -8 * wide.grad.double().abs().sum(0).max()
+
+
+@pytest.mark.parametrize("n,hw", [(0, 16), (2, 0)])
+@pytest.mark.parametrize("grad", [False, True])
+def test_group_norm_of_nothing_is_an_error(n, hw, grad):
+    with pytest.raises(RuntimeError):
+        F.group_norm_silu(mk(n, hw, 64).requires_grad_(grad), mk(64), mk(64), 8)
