@@ -67,13 +67,16 @@ class GatherJob(C.Structure):
 
 _P, _I, _L, _F, _U64, _U32 = C.c_void_p, C.c_int, C.c_longlong, C.c_float, C.c_ulonglong, C.c_uint
 
+# Kernel families with bounded waits: each has a device error word, read and cleared by eri_<family>_check_error.
+ERROR_FAMILIES = ("gemm", "gemm2", "gemm_few", "gemm_skinny", "gemm_tokred", "fa", "fa2", "fa_wide", "fa_bias", "fa_bwd", "norm")
+
 _SIGNATURES = {
+    **{f"eri_{f}_check_error": [] for f in ERROR_FAMILIES},
     "eri_norm_modulate_fwd": [_P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _F, _I, _P],
     "eri_norm_modulate_bwd": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "eri_norm_modulate_fwd_warp": [_P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _F, _I, _P],
     "eri_norm_modulate_bwd_warp": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "eri_norm_modulate_bwd_warp_add": [_P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
-    "eri_norm_check_error": [],
     "eri_norm_set_row_cta_rows": [_I],
     "eri_norm_set_smem_variant": [C.c_int],
     "eri_adamw8bit_set_pair_variant": [C.c_int],
@@ -108,20 +111,15 @@ _SIGNATURES = {
     "eri_dequant_int8": [_P, _P, _P, _L, _I, _P],
     "eri_dequant_4bit": [_P, _P, _P, _L, _I, _I, _P],
     "eri_gemm_skinny": [_P, _L, _P, _L, _P, _I, _I, _I, _I, _F, _P],
-    "eri_gemm_skinny_check_error": [],
     "eri_gemm_rank_stream": [_P, _L, _P, _L, _P, _I, _I, _I, _I, _F, _P],
     "eri_gemm_rank_stream2": [_P, _L, _P, _L, _P, _I, _I, _F, _P, _L, _P, _L, _P, _I, _I, _F, _I, _I, _P],
     "eri_gemm_tokred": [_P, _L, _P, _L, _P, _I, _I, _I, _I, _F, _I, _I, _L, _P],
-    "eri_gemm_tokred_check_error": [],
     "eri_gemm_tokred_set_target": [_I],
     "eri_gemm_init": [],
-    "eri_gemm_check_error": [],
     "eri_gemm_bf16": [C.POINTER(GemmArgs), _P],
     "eri_gemm2_bf16": [C.POINTER(GemmArgs), _P],
     "eri_gemm_few_bf16": [C.POINTER(GemmArgs), _P],
-    "eri_gemm_few_check_error": [],
     "eri_gemm2_bf16_group2": [C.POINTER(GemmArgs), C.POINTER(GemmArgs), _P],
-    "eri_gemm2_check_error": [],
     "eri_gemm2_gather_count": [],
     "eri_rows_wgrad": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _F, _P],
     "eri_rows_dgrad": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _P],
@@ -206,6 +204,13 @@ def require():
             f"native kernel library {_LIB_PATH} is missing or failed to load; run "
             "`python -m eridiffusion_b200.csrc.build` (needs nvcc) before using CUDA tensors")
     return h
+
+
+def error_words(families=ERROR_FAMILIES) -> dict:
+    """Synchronise and read the error words of ``families``: {family: word} of those that are set."""
+    h = require()
+    words = {f: getattr(h, f"eri_{f}_check_error")() for f in families}
+    return {f: w for f, w in words.items() if w}
 
 
 def ops():

@@ -26,11 +26,6 @@ N._SIGNATURES.update({
     "eri_flash_attn_fwd_masked": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _P],
     "eri_flash_attn_bwd_masked": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _P],
     "eri_flash_attn_fwd_pair": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P],
-    "eri_fa_check_error": [],
-    "eri_fa2_check_error": [],
-    "eri_fa_wide_check_error": [],
-    "eri_fa_bias_check_error": [],
-    "eri_fa_bwd_check_error": [],
 })
 
 _LOG2E = 1.4426950408889634
@@ -41,8 +36,7 @@ _MASKED = -1.0e30      # bias of a masked key: its probability is exactly zero, 
 def _bind(lib):
     for name in ("eri_flash_attn_fwd", "eri_flash_attn_bwd", "eri_flash_attn_fwd_ld", "eri_flash_attn_bwd_ld",
                  "eri_flash_attn_fwd_masked",
-                 "eri_flash_attn_bwd_masked", "eri_flash_attn_fwd_pair", "eri_fa_check_error",
-                 "eri_fa2_check_error", "eri_fa_wide_check_error", "eri_fa_bias_check_error", "eri_fa_bwd_check_error"):
+                 "eri_flash_attn_bwd_masked", "eri_flash_attn_fwd_pair"):
         if hasattr(lib, name):
             fn = getattr(lib, name)
             fn.argtypes = N._SIGNATURES[name]
@@ -254,18 +248,8 @@ def bwd(do, q, k, v, out, lse, scale=None, kbias=None):
 
 
 def check_error() -> int:
-    lib = N.require()
-    _bind(lib)
-    e = lib.eri_fa_check_error()
-    if not e and hasattr(lib, "eri_fa2_check_error"):
-        e = lib.eri_fa2_check_error()
-    if not e and hasattr(lib, "eri_fa_wide_check_error"):
-        e = lib.eri_fa_wide_check_error()
-    if not e and hasattr(lib, "eri_fa_bias_check_error"):
-        e = lib.eri_fa_bias_check_error()
-    if not e and hasattr(lib, "eri_fa_bwd_check_error"):
-        e = lib.eri_fa_bwd_check_error()
-    return e
+    """Synchronise and return the first error word that is set among the attention kernels' (0 = clean)."""
+    return next(iter(N.error_words([f for f in N.ERROR_FAMILIES if f.startswith("fa")]).values()), 0)
 
 
 class _IntoBuffer(torch.autograd.Function):

@@ -382,27 +382,13 @@ def set_gemm_pair(on: bool) -> None:
 
 def gemm_error_check() -> int:
     """Synchronise and return the device error word of the GEMM kernels (0 = clean)."""
-    lib = N.require()
-    e = lib.eri_gemm_check_error()
-    if not e and hasattr(lib, "eri_gemm2_check_error"):
-        e = lib.eri_gemm2_check_error()
-    if not e and hasattr(lib, "eri_gemm_few_check_error"):
-        e = lib.eri_gemm_few_check_error()
-    return e
+    return next(iter(N.error_words(("gemm", "gemm2", "gemm_few")).values()), 0)
 
 
 def kernel_error_check() -> dict:
     """Synchronise and read every kernel family's device error word (each is set when one of that
     family's bounded waits ran out, and cleared by the read). Empty dict = clean."""
-    lib = N.require()
-    out = {}
-    for name in ("gemm", "gemm2", "gemm_skinny", "gemm_tokred", "fa", "fa2", "fa_bwd", "norm"):
-        fn = getattr(lib, f"eri_{name}_check_error", None)
-        if fn is not None:
-            v = fn()
-            if v:
-                out[name] = v
-    return out
+    return N.error_words()
 
 
 def _wgrad_ok(*ts) -> bool:
