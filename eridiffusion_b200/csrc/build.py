@@ -123,6 +123,11 @@ def build_host(verbose: bool = False) -> Path:
     return out
 
 
+def torch_headers() -> list[Path]:
+    """The headers that the op layer may include: its own and those it shares with the kernels."""
+    return sorted((CSRC / "torch").glob("*.h")) + sorted(CSRC.glob("*.h"))
+
+
 def build_torch(verbose: bool = False) -> Path:
     """The op layer of ``torch/*.cpp`` as an extension module (one ``g++ -c`` per file, in parallel)."""
     import sysconfig
@@ -137,7 +142,7 @@ def build_torch(verbose: bool = False) -> Path:
              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-isystem", str(root / "include"),
              "-isystem", str(root / "include/torch/csrc/api/include"), "-isystem", f"{cuda_home}/include",
              "-isystem", sysconfig.get_paths()["include"]]
-    headers = b"".join(h.read_bytes() for h in (CSRC / "torch" / "eri_ops.h", CSRC / "gemm_args.h"))
+    headers = b"".join(h.read_bytes() for h in torch_headers())
 
     def compile_one(src: Path):
         obj, stamp = OBJ_DIR / f"torch_{src.stem}.o", OBJ_DIR / f"torch_{src.stem}.sha"
