@@ -130,6 +130,14 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         if (!mbar_wait(&full[stage], phase)) {
           atomicExch(p.err, 42);
           ok = false;
+          // the copies behind this one may still be on their way into this CTA's shared memory
+          for (int s = 1; s < STAGES && i + s < steps; ++s) {
+            if (++stage == STAGES) {
+              stage = 0;
+              phase ^= 1;
+            }
+            mbar_wait(&full[stage], phase);
+          }
           break;
         }
         tc_fence_after();
@@ -171,6 +179,9 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         for (int i = 0; i < 8; ++i)
           *reinterpret_cast<uint4*>(row + c * 32 + i * 4) = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
       }
+    } else {
+      // the tile becomes NaN, never what the shared memory happened to hold
+      for (int i = 0; i < 64; ++i) row[i] = __int_as_float(0x7fffffff);
     }
     tc_fence_before();
   }
