@@ -2,6 +2,8 @@
 // autograd nodes over the kernels.
 #include "eri_ops.h"
 
+#include <ATen/cuda/CUDAGraphsUtils.cuh>
+
 #include <map>
 #include <mutex>
 
@@ -372,27 +374,28 @@ Tensor glu(const Tensor& h, int mode, bool act_first) {
 namespace {
 
 // Key bias (log2 units) that blanks the padding of a key set shorter than one tile: [B, 128] rows followed by one
-// flag per (batch, tile), all set. Constant per (B, Lk, device), so kept (at most kMaxPad of them).
+// flag per (batch, tile), all set. Constant per (B, Lk, device): the first kMaxPad shapes are made once and kept for
+// good (any stream may be reading one, so none is ever given back); later shapes, and shapes first met while a graph
+// is captured, are made by the call on its own stream (three small launches).
+Tensor make_pad_bias(int64_t B, int64_t Lk, const Tensor& like) {
+  Tensor t = at::full({B * 128 + B}, -1.0e30f, like.options().dtype(at::kFloat));
+  t.narrow(0, 0, B * 128).view({B, 128}).narrow(1, 0, Lk).zero_();
+  t.narrow(0, B * 128, B).view(at::kInt).fill_(1);
+  return t;
+}
 Tensor pad_bias(int64_t B, int64_t Lk, const Tensor& like) {
   constexpr size_t kMaxPad = 64;
   static std::mutex mu;
   static std::map<std::tuple<int64_t, int64_t, int>, Tensor> cache;
   const auto key = std::make_tuple(B, Lk, (int)like.device().index());
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = cache.find(key);
-    if (it != cache.end()) return it->second;
-  }
-  Tensor host = at::empty({B * 128 + B}, at::TensorOptions().dtype(at::kFloat));
-  float* p = host.data_ptr<float>();
-  for (int64_t b = 0; b < B; ++b)
-    for (int64_t i = 0; i < 128; ++i) p[b * 128 + i] = i < Lk ? 0.f : -1.0e30f;
-  const int32_t one = 1;
-  for (int64_t b = 0; b < B; ++b) memcpy(p + B * 128 + b, &one, 4);
-  Tensor t = host.to(like.device());      // waits for the copy: any stream may read it afterwards
   std::lock_guard<std::mutex> lock(mu);
-  if (cache.size() >= kMaxPad) cache.clear();
-  cache[key] = t;
+  auto it = cache.find(key);
+  if (it != cache.end()) return it->second;
+  Tensor t = make_pad_bias(B, Lk, like);
+  if (cache.size() < kMaxPad && at::cuda::currentStreamCaptureStatus() == at::cuda::CaptureStatus::None) {
+    c10::cuda::getCurrentCUDAStream().synchronize();      // another stream may read it from now on
+    cache[key] = t;
+  }
   return t;
 }
 
