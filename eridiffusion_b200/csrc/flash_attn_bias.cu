@@ -22,7 +22,7 @@ namespace {
 
 struct BiasParams {
   int B, H, Lq, Lk;
-  float scale_log2;
+  float scale;
   bf16* out;              // [B, Lq, H, DH] contiguous
   const void* bias;       // element (b, h, q, k) at b * sb + h * sh + q * sq + k
   long long sb, sh, sq;
@@ -31,11 +31,12 @@ struct BiasParams {
 };
 
 constexpr int BQ = 128, BKV = 128;
-constexpr float kRescaleThreshold = 8.0f, kLog2e = 1.4426950408889634f;
+constexpr float kRescaleThreshold = 5.5452f /* 8 ln 2 */, kLog2e = 1.4426950408889634f;
 
 ERI_DEBUG_BOUNDS_DEFINE(fa_bias)
 
-// z[i] = s[i] * scale + bias[k0 + i] (log2 units) for 32 keys; keys at or beyond Lk are -inf.
+// z[i] = s[i] * scale + bias[k0 + i] for 32 keys; keys at or beyond Lk are -inf. In natural units, not in those of exp2:
+// a mask of the type's lowest value is finite, and times log2(e) it would not be.
 __device__ __forceinline__ void biased32(const BiasParams& p, const void* brow, int k0, const uint32_t (&r)[32], float (&z)[32]) {
   if (p.vec && k0 + 32 <= p.Lk) {
     const bf16x8* b8 = reinterpret_cast<const bf16x8*>(static_cast<const bf16*>(brow) + k0);
@@ -44,7 +45,7 @@ __device__ __forceinline__ void biased32(const BiasParams& p, const void* brow, 
       float b[8];
       unpack8(b8[g], b);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) z[g * 8 + i] = fmaf(__uint_as_float(r[g * 8 + i]), p.scale_log2, b[i] * kLog2e);
+      for (int i = 0; i < 8; ++i) z[g * 8 + i] = fmaf(__uint_as_float(r[g * 8 + i]), p.scale, b[i]);
     }
   } else {
 #pragma unroll
@@ -52,8 +53,8 @@ __device__ __forceinline__ void biased32(const BiasParams& p, const void* brow, 
       float b = -INFINITY;
       if (k0 + i < p.Lk)
         b = p.is_bool ? (static_cast<const uint8_t*>(brow)[k0 + i] ? 0.f : -INFINITY)
-                      : __bfloat162float(static_cast<const bf16*>(brow)[k0 + i]) * kLog2e;
-      z[i] = b == -INFINITY ? b : fmaf(__uint_as_float(r[i]), p.scale_log2, b);
+                      : __bfloat162float(static_cast<const bf16*>(brow)[k0 + i]);
+      z[i] = b == -INFINITY ? b : fmaf(__uint_as_float(r[i]), p.scale, b);
     }
   }
 }
@@ -193,7 +194,7 @@ fa_bias_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (__any_sync(0xffffffffu, need)) {
           // s_full of this tile was committed after the products of the previous one: O is complete
           const float m_t = need ? m_new : m_used;
-          const float alpha = need ? exp2f(m_used - m_t) : 1.f;
+          const float alpha = need ? exp2f((m_used - m_t) * kLog2e) : 1.f;
 #pragma unroll 1
           for (int c = 0; c < DH / 64; ++c) {
             uint32_t r[32];
@@ -225,7 +226,7 @@ fa_bias_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         uint32_t hi[16], lo[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          const float p0 = ex2_mufu(z[2 * i] - m_sub), p1 = ex2_mufu(z[2 * i + 1] - m_sub);
+          const float p0 = ex2_mufu((z[2 * i] - m_sub) * kLog2e), p1 = ex2_mufu((z[2 * i + 1] - m_sub) * kLog2e);
           l += p0 + p1;
           hi[i] = pack_bf162(p0, p1);
           const float2 f = bf162_bits_to_float2(hi[i]);
@@ -334,7 +335,7 @@ int eri_flash_attn_bias_fwd(const void* q, const void* k, const void* v, void* o
   if (make_map(&tq, q, B, Lq, H, DH, s.q) || make_map(&tk, k, B, Lk, H, DH, s.k) || make_map(&tv, v, B, Lk, H, DH, s.v)) return -4;
   BiasParams p;
   p.B = B; p.H = H; p.Lq = Lq; p.Lk = Lk;
-  p.scale_log2 = scale * kLog2e;
+  p.scale = scale;
   p.out = (bf16*)out; p.bias = bias; p.sb = sb; p.sh = sh; p.sq = sq; p.is_bool = is_bool; p.err = g_bias_err[dev];
   p.vec = !is_bool && sb % 8 == 0 && sh % 8 == 0 && sq % 8 == 0 && ((uintptr_t)bias & 15) == 0;
   cudaStream_t st = (cudaStream_t)stream;
