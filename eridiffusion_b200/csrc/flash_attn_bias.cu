@@ -3,10 +3,12 @@
 // relative-position bias of T5-style encoders, the causal mask of CLIP-style ones. No gradient.
 //
 // The scores, the bias sum, the exponentials and the row sums are fp32, and a probability enters the second product
-// as two bf16 terms (its rounding and the rest of it): 16 bits of mantissa, as far from fp32 as the fp32 accumulation
-// of the product itself. One CTA per (128 queries, head, batch), two per SM, as flash_attn.cu:
+// as three bf16 terms (its rounding, the rounding of the rest, and what is left): all 24 bits of its mantissa, so the
+// product is that of fp32 probabilities. One CTA per (128 queries, head, batch), two per SM at head size 64, as
+// flash_attn.cu:
 //   warp 0     TMA: Q once, then one K and one V tile of 128 keys per iteration
-//   warp 1     tcgen05.mma issue: S = Q K^T, O += P_hi V, O += P_lo V (both halves of P lie over S in TMEM)
+//   warp 1     tcgen05.mma issue: S = Q K^T, O += P1 V, O += P2 V, O += P3 V (P1 and P2 lie over S in TMEM, P3 has 64
+//              columns of its own)
 //   warps 2-9  softmax, two threads per query row, 64 keys of a tile each
 // What bounds it: latency. At 256 tokens x 64 heads 128 CTAs run two tiles each, and a thread's bias row of 64 keys is
 // one 128-byte line. The library ran this as fp32 products on the CUDA cores with separate bias, masking, softmax
@@ -65,7 +67,7 @@ fa_bias_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                    const __grid_constant__ CUtensorMap tmV, const BiasParams p) {
   constexpr int CHUNKS = DH / 64;
   constexpr int CHUNK_BYTES = 128 * 128, TILE_BYTES = CHUNK_BYTES * CHUNKS;
-  constexpr uint32_t S_COL = 0, O_COL = 128;
+  constexpr uint32_t S_COL = 0, O_COL = 128, P3_COL = O_COL + DH, TMEM = DH == 64 ? 256 : 512;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
@@ -89,7 +91,7 @@ fa_bias_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     tma_prefetch_desc(&tmV);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, 256);
+    tmem_alloc(tmem_slot, TMEM);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -137,11 +139,12 @@ fa_bias_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tc_fence_after();
 #pragma unroll
         for (int kk = 0; kk < BKV / 16; ++kk) {
-          // 32 keys take the 32 columns that their scores had: 16 columns of roundings, then 16 of remainders
+          // 32 keys take the 32 columns that their scores had: 16 columns of first terms, then 16 of second ones
           const uint32_t pcol = tmem_base + S_COL + (kk >> 1) * 32 + (kk & 1) * 8;
           const uint64_t dv = umma_desc_mn128(aV + kk * 2048, CHUNK_BYTES);
           umma_bf16_ts(tmem_base + O_COL, pcol, dv, idesc_o, (j | kk) != 0);
           umma_bf16_ts(tmem_base + O_COL, pcol + 16, dv, idesc_o, true);
+          umma_bf16_ts(tmem_base + O_COL, tmem_base + P3_COL + kk * 8, dv, idesc_o, true);
         }
         umma_commit(o_done);
         umma_commit(v_empty);
@@ -223,17 +226,21 @@ fa_bias_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tmem_ld32(lane_addr + s_col + c * 32, r);
         tmem_ld_wait();
         biased32(p, brow, kbase + c * 32, r, z);
-        uint32_t hi[16], lo[16];
+        uint32_t p1[16], p2[16], p3[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          const float p0 = ex2_mufu((z[2 * i] - m_sub) * kLog2e), p1 = ex2_mufu((z[2 * i + 1] - m_sub) * kLog2e);
-          l += p0 + p1;
-          hi[i] = pack_bf162(p0, p1);
-          const float2 f = bf162_bits_to_float2(hi[i]);
-          lo[i] = pack_bf162(p0 - f.x, p1 - f.y);
+          const float a = ex2_mufu((z[2 * i] - m_sub) * kLog2e), b = ex2_mufu((z[2 * i + 1] - m_sub) * kLog2e);
+          l += a + b;
+          p1[i] = pack_bf162(a, b);
+          const float2 f = bf162_bits_to_float2(p1[i]);
+          const float a2 = a - f.x, b2 = b - f.y;      // exact, as are the remainders of the remainders
+          p2[i] = pack_bf162(a2, b2);
+          const float2 t = bf162_bits_to_float2(p2[i]);
+          p3[i] = pack_bf162(a2 - t.x, b2 - t.y);
         }
-        tmem_st16(lane_addr + s_col + c * 32, hi);
-        tmem_st16(lane_addr + s_col + c * 32 + 16, lo);
+        tmem_st16(lane_addr + s_col + c * 32, p1);
+        tmem_st16(lane_addr + s_col + c * 32 + 16, p2);
+        tmem_st16(lane_addr + P3_COL + half * 32 + c * 16, p3);
       }
       tmem_st_wait();
       tc_fence_before();
@@ -274,7 +281,7 @@ fa_bias_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   if (warp == 1) {
     __syncwarp();
-    tmem_dealloc(tmem_base, 256);
+    tmem_dealloc(tmem_base, TMEM);
   }
 }
 
