@@ -217,6 +217,8 @@ std::vector<Tensor> qknorm_rope_joint(const std::vector<OptT>& flat, const OptT&
                                       double eps) {
   std::vector<Tensor> f;
   bool grad = false;
+  const Tensor cos_t = opt(cos), sin_t = opt(sin);
+  refuse_tangents({&cos_t, &sin_t});
   for (auto& t : flat) {
     f.push_back(opt(t));
     grad |= any_grad({&f.back()});
@@ -524,6 +526,7 @@ Tensor packed_attention(const Tensor& a, const Tensor& kv, int64_t heads, double
   Tensor kbias = opt(kbias_);
   const int64_t Lk = kv.defined() ? kv.size(1) : a.size(1);
   if (!kbias.defined() && Lk < 128) kbias = pad_bias(a.size(0), Lk, a);
+  refuse_tangents({&kbias});
   if (any_grad({&a, &kv})) return PackedAttention::apply(wrap(a), wrap(kv), wrap(kbias), heads, scale);
   Parts p(contig16(a), contig16(kv), heads);
   return attn_fwd(p.q, p.k, p.v, scale, Tensor(), kbias, -1).first.flatten(2);
@@ -535,6 +538,7 @@ Tensor packed_attention(const Tensor& a, const Tensor& kv, int64_t heads, double
 Tensor attention(const Tensor& q, const Tensor& k, const Tensor& v, double scale, const OptT& kbias_, int pair_poly) {
   Tensor kbias = opt(kbias_);
   if (!kbias.defined() && k.size(1) < 128) kbias = pad_bias(k.size(0), k.size(1), q);
+  refuse_tangents({&kbias});
   if (any_grad({&q, &k, &v})) return Attention::apply(wrap(q), wrap(k), wrap(v), wrap(kbias), scale, (int64_t)pair_poly);
   return attn_fwd(packed_heads(q), packed_heads(k), packed_heads(v), scale, Tensor(), kbias, pair_poly).first;
 }
@@ -547,6 +551,7 @@ Tensor attention_kv(const Tensor& q, const Tensor& kv, int64_t heads, double sca
 
 // q, k, v [B, L, H, 512] (column blocks of wider tensors are read in place), no gradient.
 Tensor attention_wide(const Tensor& q_, const Tensor& k_, const Tensor& v_, double scale) {
+  refuse_tangents({&q_, &k_, &v_});
   const Tensor q = packed_heads(q_), k = packed_heads(k_), v = packed_heads(v_);
   const int64_t B = q.size(0), Lq = q.size(1), H = q.size(2), Lk = k.size(1);
   TORCH_CHECK_VALUE(q.size(3) == 512 && k.sizes() == v.sizes() && k.size(0) == B && k.size(2) == H && k.size(3) == 512,
@@ -563,6 +568,7 @@ Tensor attention_wide(const Tensor& q_, const Tensor& k_, const Tensor& v_, doub
 // q, k, v [B, L, H, 64 | 128] (column blocks of wider tensors are read in place) with an additive bf16 or boolean mask
 // that broadcasts to [B, H, Lq, Lk]; no gradient.
 Tensor attention_bias(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& bias, double scale) {
+  refuse_tangents({&q_, &k_, &v_, &bias});
   const Tensor q = packed_heads(q_), k = packed_heads(k_), v = packed_heads(v_);
   const int64_t B = q.size(0), Lq = q.size(1), H = q.size(2), D = q.size(3), Lk = k.size(1);
   const bool is_bool = bias.scalar_type() == at::kBool;
@@ -637,6 +643,7 @@ Tensor attention_qkv_rope(const Tensor& qkv, const Tensor& wq, const Tensor& wk,
   const int64_t D = qkv.size(2) / 3;
   TORCH_CHECK_VALUE(wq.numel() == D && wk.numel() == D && cos.dim() == 2 && cos.size(0) == qkv.size(1) && cos.size(1) * 2 == D &&
                         sin.sizes() == cos.sizes(), "attention_qkv_rope: operand sizes");
+  refuse_tangents({&wq, &wk, &cos, &sin});
   if (any_grad({&qkv})) return RopeAttention::apply(wrap(qkv), wrap(wq), wrap(wk), wrap(cos), wrap(sin), heads, eps, true);
   return RopeAttention::forward(nullptr, qkv, wq, wk, cos, sin, heads, eps, false);
 }
@@ -663,6 +670,8 @@ struct MseLoss : torch::autograd::Function<MseLoss> {
 };
 }  // namespace
 Tensor mse_loss(const Tensor& pred, const Tensor& target, const OptT& weight) {
+  const Tensor w = opt(weight);
+  refuse_tangents({&pred, &target, &w});
   return MseLoss::apply(wrap(pred), wrap(target), weight);
 }
 
@@ -990,6 +999,8 @@ Tensor single_stream(const Tensor& xm, const Tensor& x, const Tensor& gate, cons
                      int64_t heads, int flags, bool act_fwd_epilogue, bool act_bwd_epilogue) {
   const int64_t flags2 = (act_fwd_epilogue ? 1 : 0) | (act_bwd_epilogue ? 2 : 0);
   const Tensor t[] = {opt(b1), opt(b2), opt(a1), opt(bb1), opt(a2), opt(bb2), opt(qs), opt(ks)};
+  const Tensor tables[] = {opt(cos), opt(sin)};
+  refuse_tangents({&tables[0], &tables[1]});
   const bool keep = any_grad({&xm, &x, &gate, &w1, &w2, &t[0], &t[1], &t[2], &t[3], &t[4], &t[5], &t[6], &t[7]});
   if (!keep)
     return SingleStream::forward(nullptr, xm, x, gate, w1, b1, w2, b2, a1, bb1, a2, bb2, qs, ks, cos, sin,

@@ -8,6 +8,7 @@
 #pragma once
 #include <torch/extension.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/forward_grad.h>
 
 #include <atomic>
 #include <optional>
@@ -222,7 +223,17 @@ struct Args {
   }
 };
 
+// The kernels have no forward-mode derivatives. A dual tensor is refused, whether or not gradients are recorded: its
+// result would silently have no tangent.
+inline void refuse_tangents(std::initializer_list<const Tensor*> ts) {
+  if (!torch::autograd::ForwardADLevel::try_get_by_idx(0)) return;      // no dual level is open
+  for (const Tensor* t : ts)
+    TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !t->_fw_grad(0).defined(), "forward-mode differentiation of this op");
+}
+
+// Whether a node is needed for these inputs.
 inline bool any_grad(std::initializer_list<const Tensor*> ts) {
+  refuse_tangents(ts);
   if (!at::GradMode::is_enabled()) return false;
   for (const Tensor* t : ts)
     if (t->defined() && t->requires_grad()) return true;

@@ -729,9 +729,10 @@ std::vector<Tensor> linear_pair(const std::vector<OptT>& s0, double sc0, const s
   for (int i = 0; i < 8; ++i) {
     a[i] = opt(s0[i]);
     b[i] = opt(s1[i]);
+    const bool ga = any_grad({&a[i]}), gb = any_grad({&b[i]});
     if (i != Stream::res && i != Stream::gate) {
-      keep[0] |= any_grad({&a[i]});
-      keep[1] |= any_grad({&b[i]});
+      keep[0] |= ga;
+      keep[1] |= gb;
     }
   }
   return FusedLinearPair::apply(wrap(a[0]), wrap(a[1]), wrap(a[2]), wrap(a[3]), wrap(a[4]), wrap(a[5]), wrap(a[6]), wrap(a[7]), wrap(b[0]), wrap(b[1]), wrap(b[2]), wrap(b[3]), wrap(b[4]), wrap(b[5]), wrap(b[6]), wrap(b[7]),
