@@ -228,6 +228,11 @@ struct TransposePlan {
   Tensor buf, jobs;
   int64_t max_elems = 0;
   bool valid = false;
+  // matrix i is still the tensor it was made from, at the same address
+  bool current(size_t i) const {
+    const auto t = owners[i].lock();
+    return t && t->data() == key[i];
+  }
 };
 std::mutex g_tmu;
 std::vector<std::shared_ptr<TransposePlan>> g_plans;
@@ -244,8 +249,8 @@ void drop_plan(size_t i) {
 }
 void drop_dead_plans() {
   for (size_t i = g_plans.size(); i-- > 0;)
-    for (auto& w : g_plans[i]->owners)
-      if (w.expired()) {
+    for (size_t j = 0; j < g_plans[i]->key.size(); ++j)
+      if (!g_plans[i]->current(j)) {
         drop_plan(i);
         break;
       }
@@ -294,7 +299,7 @@ int prepare_lora_transposes(const std::vector<Tensor>& all) {
   return (int)mats.size();
 }
 
-// The matrices changed (optimizer step): the copies of the plan that holds the first of them are stale. With an
+// The matrices changed (optimizer step): the copies of every plan that one of them is published by are stale. With an
 // empty list every plan is.
 void invalidate_lora_transposes(const std::vector<Tensor>& mats) {
   std::lock_guard<std::mutex> lock(g_tmu);
@@ -302,9 +307,11 @@ void invalidate_lora_transposes(const std::vector<Tensor>& mats) {
     for (auto& p : g_plans) p->valid = false;
     return;
   }
-  auto it = g_published.find(mats[0].data_ptr());
-  if (it == g_published.end()) return;
-  if (auto p = it->second.first.lock()) p->valid = false;
+  for (const Tensor& m : mats) {
+    auto it = g_published.find(m.data_ptr());
+    if (it == g_published.end()) continue;
+    if (auto p = it->second.first.lock()) p->valid = false;
+  }
 }
 
 Tensor lora_transposed(const Tensor& m) {
@@ -314,7 +321,7 @@ Tensor lora_transposed(const Tensor& m) {
     if (it != g_published.end()) {
       auto p = it->second.first.lock();
       const int i = it->second.second;
-      if (p && p->valid && !p->owners[i].expired() && p->outs[i].size(0) == m.size(1) && p->outs[i].size(1) == m.size(0))
+      if (p && p->valid && p->current(i) && p->outs[i].size(0) == m.size(1) && p->outs[i].size(1) == m.size(0))
         return p->outs[i];
     }
   }

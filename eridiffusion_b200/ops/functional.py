@@ -464,10 +464,10 @@ def prepare_lora_transposes(matrices):
 
 
 def invalidate_lora_transposes(matrices=()):
-    """The adapter matrices changed (optimizer step): the published transposes of the set that ``matrices``
-    belong to (default: of every set) are stale."""
+    """The adapter matrices changed (optimizer step): the published transposes of every set that one of ``matrices``
+    belongs to (default: of every set) are stale."""
     if N._ops is not None:
-        N._ops.invalidate_lora_transposes(list(matrices[:1]))
+        N._ops.invalidate_lora_transposes(list(matrices))
 
 
 def _lora_transposed(m):
