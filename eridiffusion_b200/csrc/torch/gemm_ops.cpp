@@ -332,7 +332,7 @@ Tensor lora_transposed(const Tensor& m) {
 // type (an undefined tensor is returned then), else returned.
 Tensor col_sum(const Tensor& x2, const Tensor& p) {
   const bool acc = has_grad_buffer(p, x2.scalar_type());
-  if (rows_ok(x2) && x2.size(1) % 8 == 0 && (!acc || al16(p.grad()))) {
+  if (x2.size(0) > 0 && rows_ok(x2) && x2.size(1) % 8 == 0 && (!acc || al16(p.grad()))) {
     Tensor out = acc ? p.grad() : empty_bf16({x2.size(1)}, x2);
     check(L.eri_col_sum(x2.data_ptr(), x2.stride(0), out.data_ptr(), (int)x2.size(0), (int)x2.size(1), acc, stream()),
           "col_sum");

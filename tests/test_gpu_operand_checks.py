@@ -69,3 +69,12 @@ def test_one_embedding_for_every_sample():
 def test_group_norm_of_nothing_is_an_error(n, hw, grad):
     with pytest.raises(RuntimeError):
         F.group_norm_silu(mk(n, hw, 64).requires_grad_(grad), mk(64), mk(64), 8)
+
+
+@pytest.mark.parametrize("buffers", [False, True])
+def test_linear_without_rows_has_zero_gradients(buffers):
+    x, w, b = mk(2, 0, 64).requires_grad_(), mk(256, 64).requires_grad_(), mk(256).requires_grad_()
+    if buffers:
+        w.grad, b.grad = torch.ones_like(w), torch.ones_like(b)
+    F.linear(x, w, b).backward(mk(2, 0, 256))
+    assert x.grad.shape == x.shape and all((p.grad == (1 if buffers else 0)).all() for p in (w, b))
