@@ -405,11 +405,13 @@ Tensor pad_bias(int64_t B, int64_t Lk, const Tensor& like) {
 
 namespace {
 
-// Token stride of a [B, L, H, D] operand the kernels read or write in place (heads packed).
+// Token stride of a [B, L, H, D] operand the kernels read or write in place (heads packed), 0 where there is none. The
+// stride of a dimension of size 1 says nothing: a contiguous tensor may have any value there.
 int64_t token_stride(const Tensor& t) {
-  const int64_t ld = t.stride(1), H = t.size(2), D = t.size(3);
-  const bool ok = t.stride(3) == 1 && t.stride(2) == D && ld >= H * D && ld % 8 == 0 && al16(t) &&
-                  (t.size(0) == 1 || t.stride(0) == t.size(1) * ld);
+  const int64_t B = t.size(0), L_ = t.size(1), H = t.size(2), D = t.size(3);
+  const int64_t ld = L_ > 1 ? t.stride(1) : B > 1 ? t.stride(0) : H * D;
+  const bool ok = t.stride(3) == 1 && (H == 1 || t.stride(2) == D) && ld >= H * D && ld % 8 == 0 && al16(t) &&
+                  (B == 1 || t.stride(0) == L_ * ld);
   return ok ? ld : 0;
 }
 Tensor packed_heads(const Tensor& t) { return token_stride(t) ? t : contig16(t); }

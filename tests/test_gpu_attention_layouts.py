@@ -1,0 +1,37 @@
+"""Attention operands in every layout that callers hand over give what contiguous copies give, bit for bit, on the kernels."""
+import pytest
+import torch
+
+from eridiffusion_b200.ops import functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+def mk(*s):
+    return torch.randn(*s, device="cuda").to(torch.bfloat16)
+
+
+def same_as_contiguous(q, k, v, **kw):
+    def run(ts):
+        ts = [t.detach().requires_grad_() for t in ts]
+        n = F.ATTENTION_CALLS["native"]
+        o = F.attention(*ts, **kw)
+        assert F.ATTENTION_CALLS["native"] == n + 1
+        o.backward(do)
+        return o, [t.grad for t in ts]
+    do = mk(*q.shape)
+    o, g = run((q, k, v))
+    oc, gc = run([torch.empty(t.shape, device="cuda", dtype=t.dtype).copy_(t) for t in (q, k, v)])
+    assert torch.equal(o, oc) and all(torch.equal(a, b) for a, b in zip(g, gc))
+    with torch.no_grad():
+        assert torch.equal(F.attention(q, k, v, **kw), oc)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_dimensions_of_size_one(D):
+    one_head = [mk(2, 1, 256, D).transpose(1, 2) for _ in range(3)]
+    assert one_head[0].is_contiguous() and one_head[0].stride(2) != D
+    same_as_contiguous(*one_head)
+    same_as_contiguous(mk(2, 32, 4, D), *(mk(2, 4, 1, D).transpose(1, 2) for _ in "kv"))       # one key
+    same_as_contiguous(*(mk(256, 1, 4, D).transpose(0, 1) for _ in "qkv"))                      # one sample
+    same_as_contiguous(mk(1, 32, 1, D), *(mk(1, 1, 1, D).expand(1, 1, 1, D) for _ in "kv"))
