@@ -104,13 +104,15 @@ def pair_forward_ok(device, force: bool = False) -> bool:
     return ok
 
 
-def supported(q, k, v) -> bool:
+def supported(q, k, v, strided: bool = False) -> bool:
     """Shapes the kernels take: head size 64 / 128, at least one key, at least 16 query rows
-    (shorter query sets are conditioning-vector sized and stay on the library)."""
+    (shorter query sets are conditioning-vector sized and stay on the library). ``fwd`` and ``bwd`` want
+    contiguous operands; ``strided``: so does not ``flash_attention`` without a destination, which reads
+    column blocks of a projection in place and copies what it cannot read."""
     if not has_forward():
         return False
     B, L, H, D = q.shape
-    return (D in (64, 128) and q.is_contiguous() and k.is_contiguous() and v.is_contiguous()
+    return (D in (64, 128) and (strided or (q.is_contiguous() and k.is_contiguous() and v.is_contiguous()))
             and k.shape[1] >= 1 and L >= 16 and k.shape[2] == H and v.shape == k.shape and k.shape[0] == B)
 
 

@@ -610,7 +610,7 @@ def attention(q, k, v, scale=None, mask=None, out=None):
     if _ATTN_NATIVE == "native" and _native_ok(q, k, v):
         from . import flash_attn as FA
         # key-only masks (text padding, [B, 1, 1, T]) ride on the native kernel as a per-key bias
-        if FA.supported(q, k, v) and (mask is None or FA.mask_is_key_only(mask, q.shape[0], k.shape[1])):
+        if FA.supported(q, k, v, strided=out is None) and (mask is None or FA.mask_is_key_only(mask, q.shape[0], k.shape[1])):
             ATTENTION_CALLS["native"] += 1
             return FA.flash_attention(q, k, v, scale, out, mask)
         if mask is None and out is None and _wide_ok(q, k, v):

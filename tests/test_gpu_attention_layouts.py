@@ -35,3 +35,23 @@ def test_dimensions_of_size_one(D):
     same_as_contiguous(mk(2, 32, 4, D), *(mk(2, 4, 1, D).transpose(1, 2) for _ in "kv"))       # one key
     same_as_contiguous(*(mk(256, 1, 4, D).transpose(0, 1) for _ in "qkv"))                      # one sample
     same_as_contiguous(mk(1, 32, 1, D), *(mk(1, 1, 1, D).expand(1, 1, 1, D) for _ in "kv"))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("H", [1, 3])
+@pytest.mark.parametrize("masked", [False, True])
+def test_column_blocks_and_transposed_views(D, H, masked):
+    kw = dict(mask=torch.rand(2, 1, 1, 140, device="cuda") > 0.3) if masked else {}
+    same_as_contiguous(*mk(2, 140, 3, H, D).unbind(2), **kw)                                # a packed projection
+    same_as_contiguous(*(mk(2, H, 140, D).transpose(1, 2) for _ in "qkv"), **kw)            # head-major tensors
+    same_as_contiguous(*(mk(2, 140, H, D + 1)[..., 1:] for _ in "qkv"), **kw)               # rows that are not aligned
+    wide = mk(2, 140, H, 2 * D)
+    same_as_contiguous(wide[..., :D], mk(2, 140, H, D), wide[..., D:], **kw)
+
+
+def test_autoencoder_and_encoder_attention_stay_on_the_kernels():
+    """Callers hand over views of the packed projection: head size 64 without a mask, and with a key mask."""
+    from eridiffusion_b200.models.vae import _Attn
+    n = dict(F.ATTENTION_CALLS)
+    _Attn(64, 32, dict(device="cuda", dtype=torch.bfloat16))(mk(1, 64, 16, 16).contiguous(memory_format=torch.channels_last))
+    assert F.ATTENTION_CALLS["native"] == n["native"] + 1 and F.ATTENTION_CALLS["library"] == n["library"]
