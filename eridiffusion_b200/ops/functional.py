@@ -613,7 +613,7 @@ def attention(q, k, v, scale=None, mask=None, out=None):
         if FA.supported(q, k, v, strided=out is None) and (mask is None or FA.mask_is_key_only(mask, q.shape[0], k.shape[1])):
             ATTENTION_CALLS["native"] += 1
             return FA.flash_attention(q, k, v, scale, out, mask)
-        if mask is None and out is None and _wide_ok(q, k, v):
+        if mask is None and out is None and _wide_ok(q, k, v, scale):
             ATTENTION_CALLS["native"] += 1
             return N.ops().attention_wide(q, k, v, scale if scale is not None else 1.0 / math.sqrt(512))
         if mask is not None and out is None and _bias_ok(q, k, v, mask):
@@ -640,16 +640,22 @@ def attention(q, k, v, scale=None, mask=None, out=None):
     return R.attention(q, k, v, scale, mask)
 
 
-def _wide_ok(q, k, v) -> bool:
-    """Head size 512 (the image autoencoders' middle block), forward only: tiles of 128 queries and 128 keys."""
-    return (q.shape[-1] == 512 and q.shape[1] >= 128 and k.shape[1] >= 128 and k.shape == v.shape and q.shape[0] == k.shape[0]
+_GRID_YZ = 65535       # blocks in the second and third dimension of a launch
+
+
+def _wide_ok(q, k, v, scale) -> bool:
+    """Head size 512 (the image autoencoders' middle block), forward only: tiles of 128 queries and 128 keys. The kernel
+    takes a row's maximum before it scales, so a negative scale is the library's."""
+    return (q.shape[-1] == 512 and (scale is None or scale >= 0) and 1 <= q.shape[0] <= _GRID_YZ and 1 <= q.shape[2] <= _GRID_YZ
+            and q.shape[1] >= 128 and k.shape[1] >= 128 and k.shape == v.shape and q.shape[0] == k.shape[0]
             and q.shape[2] == k.shape[2] and not (torch.is_grad_enabled() and any(t.requires_grad for t in (q, k, v))))
 
 
 def _bias_ok(q, k, v, mask) -> bool:
     """A mask per query and key (relative-position bias, causal), forward only: bf16 or boolean, a value for every key."""
     B, Lq, H, D = q.shape
-    return (D in (64, 128) and k.shape == v.shape == (B, k.shape[1], H, D) and mask.device == q.device
+    return (D in (64, 128) and 1 <= B <= _GRID_YZ and 1 <= H <= _GRID_YZ and Lq >= 1 and k.shape[1] >= 1
+            and k.shape == v.shape == (B, k.shape[1], H, D) and mask.device == q.device
             and mask.dtype in (torch.bool, torch.bfloat16) and mask.dim() == 4 and mask.shape[3] == k.shape[1]
             and mask.shape[0] in (1, B) and mask.shape[1] in (1, H) and mask.shape[2] in (1, Lq)
             and not (torch.is_grad_enabled() and any(t.requires_grad for t in (q, k, v, mask))))

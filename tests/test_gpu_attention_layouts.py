@@ -55,3 +55,12 @@ def test_autoencoder_and_encoder_attention_stay_on_the_kernels():
     n = dict(F.ATTENTION_CALLS)
     _Attn(64, 32, dict(device="cuda", dtype=torch.bfloat16))(mk(1, 64, 16, 16).contiguous(memory_format=torch.channels_last))
     assert F.ATTENTION_CALLS["native"] == n["native"] + 1 and F.ATTENTION_CALLS["library"] == n["library"]
+
+
+@pytest.mark.parametrize("scale", [-2.0, -0.1, 0.0, 2.0])
+def test_head_512_with_any_scale(scale):
+    q, k, v = mk(1, 160, 1, 512), mk(1, 192, 1, 512), mk(1, 192, 1, 512)
+    o = F.attention(q, k, v, scale=scale)
+    r = F.R.attention_fp32(q.double(), k.double(), v.double(), scale)
+    # bf16 probabilities and one rounding of the result: 2^-8 of values of order one to four
+    assert torch.isfinite(o).all() and (o.float() - r).abs().max().item() < 2.0 ** -5
