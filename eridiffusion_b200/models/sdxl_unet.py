@@ -139,11 +139,13 @@ class ResBlock(nn.Module):
         self.skip = nn.Conv2d(cin, cout, 1, dtype=dtype, device=device) if cin != cout else None
 
     def forward(self, x, emb):
-        if F.conv_fusable(x, self.conv1, self.conv2, self.skip):
+        if F.conv_fusable(x, self.conv1, self.conv2, self.skip) and type(self.norm2) is GroupNormAct and F.unhooked(self.norm2):
             # the first convolution's bias and the time embedding are added where the second norm reads its input,
             # the other biases in the residual sum
             h = F.conv_no_bias(self.conv1, self.norm1(x))
-            h = self.norm2(h, self.conv1.bias, F.small_linear(emb, self.temb.weight, self.temb.bias, silu_in=True))
+            e = F.small_linear(emb, self.temb.weight, self.temb.bias, silu_in=True) \
+                if type(self.temb) is nn.Linear and F.unhooked(self.temb) else self.temb(TF.silu(emb))
+            h = self.norm2(h, self.conv1.bias, e)
             h = F.conv_no_bias(self.conv2, h)
             if self.skip is None:
                 return F.add_bias(x, h, self.conv2.bias)

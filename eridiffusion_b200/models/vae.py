@@ -59,7 +59,8 @@ class _Res(nn.Module):
         self.skip = nn.Conv2d(cin, cout, 1, **kw) if cin != cout else None
 
     def fusable(self, x):
-        return F.conv_fusable(x, self.c1, self.c2, self.skip)
+        return F.conv_fusable(x, self.c1, self.c2, self.skip) and type(self.n1) is type(self.n2) is _GN \
+            and F.unhooked(self.n1, self.n2)
 
     def forward(self, x, pre=None):
         """``pre`` (with ``fusable`` only): the bias [C] of the convolution that produced x, not added yet."""
@@ -86,7 +87,7 @@ def _run(blocks, h, resample, conv_in=None):
             continue
         h = h if b is conv_in else resample(h)
         nxt = blocks[i + 1] if i + 1 < len(blocks) else None
-        if type(nxt) is _Res and b.bias is not None and F.conv_fusable(h, b) and nxt.fusable(h):
+        if type(nxt) is _Res and b.bias is not None and F.unhooked(nxt) and F.conv_fusable(h, b) and nxt.fusable(h):
             h, pre = F.conv_no_bias(b, h), b.bias
         else:
             h = b(h)

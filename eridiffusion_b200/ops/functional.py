@@ -818,11 +818,18 @@ def upsample2x(x):
     return torch.nn.functional.interpolate(x, scale_factor=2.0, mode="nearest")
 
 
+def unhooked(*modules) -> bool:
+    """Whether nobody listens to these modules' calls (forward or backward hooks, a replaced ``forward``): only then may
+    their work be done without calling them, or be handed other arguments than they would see."""
+    return all(not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
+                    or "forward" in m.__dict__) for m in modules)
+
+
 def conv_fusable(x, *convs) -> bool:
     """Whether the biases of ``convs`` may be added by the ops around them (``group_norm_silu``'s ``pre_c``,
     ``add_bias``) instead of in a pass after each convolution: plain convolutions on the native path."""
-    return _native_ok(x) and all(c is None or (type(c) is torch.nn.Conv2d and not c._forward_hooks and not c._forward_pre_hooks
-                                               and c.padding_mode == "zeros" and c.out_channels % 8 == 0) for c in convs)
+    return _native_ok(x) and all(c is None or (type(c) is torch.nn.Conv2d and unhooked(c) and c.padding_mode == "zeros"
+                                               and c.out_channels % 8 == 0) for c in convs)
 
 
 def conv_no_bias(conv, x):
