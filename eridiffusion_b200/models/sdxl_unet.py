@@ -259,9 +259,11 @@ class SDXLUNet(nn.Module):
         return self.conv_out(self.norm_out(h))
 
     def samples_independent(self) -> bool:
-        """Whether two batches may share one call: no hooks, and every cross-attention is the model's own (an image
-        adapter's holds the tokens of one batch)."""
-        if self._forward_hooks or self._forward_pre_hooks:
+        """Whether two batches may share one call: nobody listens to a module's calls (a hook would see the doubled batch),
+        and every cross-attention is the model's own (an image adapter's holds the tokens of one batch)."""
+        every = torch.nn.modules.module
+        if every._global_forward_hooks or every._global_forward_pre_hooks \
+                or any(m._forward_hooks or m._forward_pre_hooks for m in self.modules()):
             return False
         blocks = [b for m in (*self.down, self.mid, *self.up) if isinstance(m, nn.ModuleList)
                   for t in m if isinstance(t, Transformer2D) for b in t.blocks]
