@@ -126,6 +126,14 @@ def channels_last_convs(model):
     return model
 
 
+def add_linear(lin, x, residual):
+    """``residual + lin(x)``: in the layer's epilogue when it is one of this package's linears (bare, adapted or quantised)
+    and nobody listens to its output, else as the sum of two tensors."""
+    if type(lin).__name__ in ("Linear", "QuantizedLinear") and hasattr(lin, "frozen_transpose") and F.unhooked(lin):
+        return lin(x, residual=residual)
+    return residual + lin(x)
+
+
 class SmallLinear(Linear):
     """Linear applied to a few conditioning rows (adaLN modulation, embedders)."""
 

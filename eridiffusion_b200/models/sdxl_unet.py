@@ -19,7 +19,7 @@ import torch.nn as nn
 import torch.nn.functional as TF
 
 from ..ops import functional as F
-from .layers import Linear, channels_last_convs, timestep_embedding
+from .layers import Linear, add_linear, channels_last_convs, timestep_embedding
 from .registry import register_model
 
 
@@ -124,7 +124,7 @@ class Transformer2D(nn.Module):
         h = self.proj_in(h)
         for blk in self.blocks:
             h = blk(h, ctx)
-        h = self.proj_out(h, residual=x.permute(0, 2, 3, 1).reshape(B, H * W, C))
+        h = add_linear(self.proj_out, h, x.permute(0, 2, 3, 1).reshape(B, H * W, C))
         return h.view(B, H, W, C).permute(0, 3, 1, 2)
 
 

@@ -18,7 +18,7 @@ import torch.nn as nn
 import torch.nn.functional as TF
 
 from ..ops import functional as F
-from .layers import Linear, rope_table
+from .layers import Linear, add_linear, rope_table
 from .registry import register_model
 
 
@@ -145,8 +145,8 @@ class _T5Layer(nn.Module):
         q, k, v = self.qkv(self.ln1(x)).view(B, T, 3, self.heads, self.head_dim).unbind(2)
         # T5 attention is unscaled and carries an additive relative-position bias
         o = F.attention(q, k, v, scale=1.0, mask=bias)
-        x = self.o(o.reshape(B, T, -1), residual=x)
-        return self.wo(F.glu(self.wi(self.ln2(x)), "gelu", act_first=True), residual=x)
+        x = add_linear(self.o, o.reshape(B, T, -1), x)
+        return add_linear(self.wo, F.glu(self.wi(self.ln2(x)), "gelu", act_first=True), x)
 
 
 class T5Encoder(nn.Module):
