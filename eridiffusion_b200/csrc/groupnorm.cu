@@ -37,7 +37,8 @@ struct GnArgs {
   float eps;
 };
 
-constexpr int kUnroll = 4, kMaxThreads = 640;    // up to 5120 channels
+// A thread per eight channels at least: 640 threads up to 5120 channels, 1024 (and half the registers) up to 8192.
+constexpr int kUnroll = 4, kMaxThreads = 640, kWideThreads = 1024;
 // Partial records an apply CTA adds itself; more are folded by a launch of their own, because every apply CTA
 // re-reads all of them (64 records of 32 groups: 16 KB from L2, about a microsecond).
 constexpr int kMaxDirectChunks = 64;
@@ -73,8 +74,8 @@ __device__ __forceinline__ void load_pre(const GnArgs& a, int n, int v, float (&
   }
 }
 
-template <bool BWD, bool PRE>
-__global__ void __launch_bounds__(kMaxThreads) gn_column_kernel(const GnArgs a) {
+template <bool BWD, bool PRE, int THREADS>
+__global__ void __launch_bounds__(THREADS) gn_column_kernel(const GnArgs a) {
   constexpr int S = BWD && PRE ? 3 : 2;
   extern __shared__ float sm[];     // [R][C][S] partial sums of the CTA's row lanes
   const int n = blockIdx.y, nvec = a.C >> 3;
@@ -178,10 +179,19 @@ __global__ void __launch_bounds__(kMaxThreads) gn_column_kernel(const GnArgs a) 
   }
 }
 
-// Many chunks: their group records folded into one (one CTA per sample).
+// Many chunks: their group records folded into one (one CTA per sample; several lanes per record word, or with more than
+// 512 groups several words per thread).
 __global__ void gn_fold_kernel(GnArgs a, float* folded) {
   const int n = blockIdx.x, lanes = blockDim.x / (2 * a.G);
   extern __shared__ float sm[];     // [lanes][2 * G]
+  if (lanes == 0) {
+    for (int i = threadIdx.x; i < 2 * a.G; i += blockDim.x) {
+      float v = 0.f;
+      for (int c = 0; c < a.chunks; ++c) v += a.part[((size_t)n * a.chunks + c) * a.G * 2 + i];
+      folded[(size_t)n * a.G * 2 + i] = v;
+    }
+    return;
+  }
   const int i = threadIdx.x % (2 * a.G), l = threadIdx.x / (2 * a.G);
   const float* p = a.part + (size_t)n * a.chunks * a.G * 2;
   if (l < lanes) {
@@ -247,8 +257,8 @@ __device__ __forceinline__ void param_gradients(const GnArgs& a, int cta, float*
   }
 }
 
-template <bool BWD, bool PRE>
-__global__ void __launch_bounds__(kMaxThreads) gn_apply_kernel(const GnArgs a) {
+template <bool BWD, bool PRE, int THREADS>
+__global__ void __launch_bounds__(THREADS) gn_apply_kernel(const GnArgs a) {
   extern __shared__ float sm[];     // [2 * G]; parameter CTAs [threads / 32][32][5]
   const int nvec = a.C >> 3;
   if (BWD && (int)blockIdx.x >= a.apply_ctas) {
@@ -372,10 +382,9 @@ GnPlan plan_for(int N, int HW, int C) {
   return p;
 }
 
-template <bool BWD, bool PRE>
+template <bool BWD, bool PRE, int THREADS>
 int run_v(GnArgs a, float* ws, cudaStream_t st) {
   const GnPlan p = plan_for(a.N, a.HW, a.C);
-  if (p.threads > kMaxThreads || 2 * a.G > 1024) return -1;
   a.chunks = a.gchunks = p.chunks;
   a.rows_per_chunk = p.rows_per_chunk;
   a.apply_ctas = p.apply_ctas;
@@ -388,15 +397,15 @@ int run_v(GnArgs a, float* ws, cudaStream_t st) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -2;
   if (!configured[dev]) {
-    if (cudaFuncSetAttribute(gn_column_kernel<BWD, PRE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kMaxThreads * 8 * S * (int)sizeof(float)) != cudaSuccess)
+    if (cudaFuncSetAttribute(gn_column_kernel<BWD, PRE, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             THREADS * 8 * S * (int)sizeof(float)) != cudaSuccess)
       return -2;
     configured[dev] = true;
   }
-  gn_column_kernel<BWD, PRE><<<dim3(p.chunks, a.N), p.threads, smem, st>>>(a);
+  gn_column_kernel<BWD, PRE, THREADS><<<dim3(p.chunks, a.N), p.threads, smem, st>>>(a);
   if (p.chunks > kMaxDirectChunks) {
-    const int lanes = 1024 / (2 * a.G) < 1 ? 1 : 1024 / (2 * a.G);
-    gn_fold_kernel<<<a.N, lanes * 2 * a.G, lanes * 2 * a.G * sizeof(float), st>>>(a, folded);
+    const int lanes = 1024 / (2 * a.G), threads = lanes ? lanes * 2 * a.G : 1024;
+    gn_fold_kernel<<<a.N, threads, threads * sizeof(float), st>>>(a, folded);
     a.part = folded;
     a.gchunks = 1;
   }
@@ -404,12 +413,16 @@ int run_v(GnArgs a, float* ws, cudaStream_t st) {
   const int extra = params ? (a.C + 31) / 32 : 0;
   int smem_apply = 2 * a.G * (int)sizeof(float);
   if (params && p.threads * 5 * (int)sizeof(float) > smem_apply) smem_apply = p.threads * 5 * (int)sizeof(float);
-  gn_apply_kernel<BWD, PRE><<<dim3(p.apply_ctas + extra, a.N), p.threads, smem_apply, st>>>(a);
+  gn_apply_kernel<BWD, PRE, THREADS><<<dim3(p.apply_ctas + extra, a.N), p.threads, smem_apply, st>>>(a);
   return (int)cudaGetLastError();
 }
 template <bool BWD>
 int run(const GnArgs& a, float* ws, cudaStream_t st) {
-  return a.pre_c || a.pre_nc ? run_v<BWD, true>(a, ws, st) : run_v<BWD, false>(a, ws, st);
+  const int threads = plan_for(a.N, a.HW, a.C).threads;
+  if (threads > kWideThreads || a.G > 4096) return -1;
+  const bool pre = a.pre_c || a.pre_nc;
+  if (threads > kMaxThreads) return pre ? run_v<BWD, true, kWideThreads>(a, ws, st) : run_v<BWD, false, kWideThreads>(a, ws, st);
+  return pre ? run_v<BWD, true, kMaxThreads>(a, ws, st) : run_v<BWD, false, kMaxThreads>(a, ws, st);
 }
 
 }  // namespace

@@ -777,7 +777,7 @@ def group_norm_silu(x, weight, bias=None, groups=32, eps=1e-5, silu=True, pre_c=
     same logical shape and format). ``pre_c`` [C] and ``pre_nc`` [N, C] are added to x before the norm (the
     bias of the convolution that produced x and a per-sample embedding), in the same pass on the native path."""
     C = x.shape[1] if x.dim() == 4 else x.shape[-1]
-    if _native_ok(x, weight, bias, pre_c, pre_nc) and C % 8 == 0 and C % groups == 0 and C <= 5120 and groups <= 512:
+    if _native_ok(x, weight, bias, pre_c, pre_nc) and C % 8 == 0 and C % groups == 0 and C <= 8192 and groups <= 4096:
         return N.ops().group_norm_silu(x, weight, bias, pre_c, pre_nc, groups, eps, silu)
     nchw = x.dim() == 4
     if nchw:
