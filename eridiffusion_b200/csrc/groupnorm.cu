@@ -271,7 +271,8 @@ __global__ void __launch_bounds__(THREADS) gn_apply_kernel(const GnArgs a) {
   if constexpr (!BWD) {
     for (int g = threadIdx.x; g < a.G; g += blockDim.x) {
       const float mean = sm[2 * g] * inv_m;
-      const float rstd = rsqrtf(fmaxf(sm[2 * g + 1] * inv_m - mean * mean, 0.f) + a.eps);
+      const float var = sm[2 * g + 1] * inv_m - mean * mean;      // inf - inf where the squares overflow: stays NaN
+      const float rstd = rsqrtf((var < 0.f ? 0.f : var) + a.eps);
       sm[2 * g] = mean;
       sm[2 * g + 1] = rstd;
       if (blockIdx.x == 0 && a.mean) {

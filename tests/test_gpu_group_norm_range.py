@@ -35,3 +35,14 @@ def test_wide_and_many_groups(Nn, HW, C, G, pre):
         scale = leaves[0].grad.abs().sum(1).max().item()
         assert (pn.grad.float() - leaves[4].grad).abs().max().item() <= 1e-2 * scale
         assert (pc.grad.float() - leaves[3].grad).abs().max().item() <= 1e-2 * Nn * scale
+
+
+@pytest.mark.parametrize("value", [1e20, -3e30, float("inf"), float("nan")])
+def test_overflowing_groups_are_not_finite_garbage(value):
+    """Squares beyond fp32's range cannot be normalised: NaN, never a finite value; the other groups are untouched."""
+    x = rnd(1, 64, 256, seed=1)
+    w, b = torch.ones(256, device="cuda").bfloat16(), torch.zeros(256, device="cuda").bfloat16()
+    clean = F.group_norm_silu(x, w, b, 32, silu=False)
+    x[..., :8] = value
+    y = F.group_norm_silu(x, w, b, 32, silu=False)
+    assert y[..., :8].isnan().all() and torch.equal(y[..., 8:], clean[..., 8:])
