@@ -53,18 +53,18 @@ NormOut norm_forward(const Tensor& x_, const Tensor& scale_, const Tensor& shift
 // is added to dx inside the backward kernel instead of by a separate autograd sum.
 struct NormModulate : torch::autograd::Function<NormModulate> {
   static variable_list forward(AutogradContext* ctx, const OptT& x_o, const OptT& scale_o, const OptT& shift_o,
-                               const OptT& weight_o, const OptT& bias_o, double eps, bool rms, bool skip) {
+                               const OptT& weight_o, const OptT& bias_o, double eps, bool rms, bool skip, bool accum) {
     const Tensor x = opt(x_o), scale = opt(scale_o), shift = opt(shift_o), weight = opt(weight_o), bias = opt(bias_o);
     if (ctx) ctx->saved_data["args"] = Args({&x, &scale, &shift, &weight, &bias}).mask;
     NormOut r = norm_forward(x, scale, shift, weight, bias, eps, rms);
     ctx->save_for_backward({r.x, r.scale, weight, bias, r.mean, r.rstd});
-    ctx->saved_data["m"] = std::vector<int64_t>{r.stride, rms, skip};
+    ctx->saved_data["m"] = std::vector<int64_t>{r.stride, rms, skip, accum};
     ctx->set_materialize_grads(false);
     if (skip) return {r.y, r.x.view(r.x.sizes())};
     return {r.y};
   }
   static variable_list backward(AutogradContext* ctx, variable_list gout) {
-    variable_list out(8);
+    variable_list out(9);
     const auto m = ctx->saved_data["m"].toIntVector();
     Tensor dskip = m[2] ? gout[1] : Tensor();
     if (!gout[0].defined()) {       // the consumer had no gradient for this input (an unused stream)
@@ -102,7 +102,7 @@ struct NormModulate : torch::autograd::Function<NormModulate> {
           if (want_sh) out[2] = d0 = empty_bf16({B, D}, x);
           if (want_sc) out[1] = d1 = empty_bf16({B, D}, x);
         } else {
-          const bool acc_b = want_b && has_grad_buffer(bias, at::kBFloat16), acc_w = want_w && has_grad_buffer(weight, at::kBFloat16);
+          const bool acc_b = want_b && has_grad_buffer(bias, at::kBFloat16, m[3]), acc_w = want_w && has_grad_buffer(weight, at::kBFloat16, m[3]);
           if (want_b) d0 = acc_b ? bias.grad() : (out[4] = empty_bf16({D}, x));
           if (want_w) d1 = acc_w ? weight.grad() : (out[3] = empty_bf16({D}, x));
           acc = (acc_b ? 1 : 0) | (acc_w ? 2 : 0);
@@ -127,9 +127,9 @@ struct NormModulate : torch::autograd::Function<NormModulate> {
 }  // namespace
 
 std::vector<Tensor> norm_modulate(const Tensor& x, const OptT& scale_, const OptT& shift_, const OptT& weight_,
-                                  const OptT& bias_, double eps, bool rms, bool skip) {
+                                  const OptT& bias_, double eps, bool rms, bool skip, bool accum) {
   Tensor scale = opt(scale_), shift = opt(shift_), weight = opt(weight_), bias = opt(bias_);
-  if (any_grad({&x, &scale, &shift, &weight, &bias})) return NormModulate::apply(wrap(x), wrap(scale), wrap(shift), wrap(weight), wrap(bias), eps, rms, skip);
+  if (any_grad({&x, &scale, &shift, &weight, &bias})) return NormModulate::apply(wrap(x), wrap(scale), wrap(shift), wrap(weight), wrap(bias), eps, rms, skip, accum);
   Tensor y = norm_forward(x, scale, shift, weight, bias, eps, rms).y;
   if (skip) return {y, x};
   return {y};
@@ -712,13 +712,13 @@ Tensor gn_forward(const Tensor& x, const Tensor& w, const Tensor& b, const Tenso
 }
 struct GroupNormSilu : torch::autograd::Function<GroupNormSilu> {
   static Tensor forward(AutogradContext* ctx, const OptT& x_o, const OptT& w_o, const OptT& b_o, const OptT& pc_o,
-                        const OptT& pn_o, int64_t groups, double eps, bool silu) {
+                        const OptT& pn_o, int64_t groups, double eps, bool silu, bool accum) {
     const Tensor x = rows_contig(*x_o), w = contig16(*w_o), b = contig16(opt(b_o)), pc = contig16(opt(pc_o)), pn = contig16(opt(pn_o));
     ctx->saved_data["args"] = Args({&x, &w, &b, &pc, &pn}).mask;
     Tensor stats = empty_f32({2, x.size(0), groups}, x);
     Tensor y = gn_forward(x, w, b, pc, pn, groups, eps, silu, stats);
     ctx->save_for_backward({x, w, b, stats, pc, pn});
-    ctx->saved_data["m"] = std::vector<int64_t>{groups, silu};
+    ctx->saved_data["m"] = std::vector<int64_t>{groups, silu, accum};
     return y;
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
@@ -730,11 +730,11 @@ struct GroupNormSilu : torch::autograd::Function<GroupNormSilu> {
     Tensor dy = rows_contig(g[0]), dx = at::empty_like(x), ws = empty_f32({L.eri_gn_workspace(r.N, r.HW, r.C, G, 1)}, x);
     const Args args(ctx->saved_data["args"].toInt());
     // a parameter's gradient goes straight into its buffer when it has one
-    variable_list out(8);
+    variable_list out(9);
     int acc = 0;
     auto dest = [&](int arg, const Tensor& p, int bit) -> void* {
       if (!args.need(ctx, arg)) return nullptr;
-      if (has_grad_buffer(p, at::kBFloat16)) {
+      if (has_grad_buffer(p, at::kBFloat16, m[2])) {
         acc |= bit;
         return p.grad().data_ptr();
       }
@@ -767,19 +767,20 @@ Tensor as_matrix(const Tensor& x) {
   return x.dim() == 4 ? x.permute({0, 2, 3, 1}).view({(int64_t)r.N * r.HW, r.C}) : x.view({(int64_t)r.N * r.HW, r.C});
 }
 struct AddBias : torch::autograd::Function<AddBias> {
-  static Tensor forward(AutogradContext* ctx, const OptT& a_o, const OptT& b_o, const OptT& bias_o, const OptT& bias2_o) {
+  static Tensor forward(AutogradContext* ctx, const OptT& a_o, const OptT& b_o, const OptT& bias_o, const OptT& bias2_o, bool accum) {
     const Tensor a = rows_contig(*a_o), b = rows_contig(*b_o), bias = contig16(opt(bias_o)), bias2 = contig16(opt(bias2_o));
     ctx->saved_data["args"] = Args({&a, &b, &bias, &bias2}).mask;
     ctx->save_for_backward({bias, bias2});
+    ctx->saved_data["accum"] = accum;
     return add_bias_forward(a, b, bias, bias2);
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     auto sv = ctx->get_saved_variables();
     const Args args(ctx->saved_data["args"].toInt());
     Tensor d = rows_contig(g[0]);
-    variable_list out{d, d, Tensor(), Tensor()};
+    variable_list out{d, d, Tensor(), Tensor(), Tensor()};
     for (int i = 0; i < 2; ++i)
-      if (args.need(ctx, 2 + i)) out[2 + i] = col_sum(as_matrix(d), sv[i]);
+      if (args.need(ctx, 2 + i)) out[2 + i] = col_sum(as_matrix(d), sv[i], ctx->saved_data["accum"].toBool());
     return out;
   }
 };
@@ -798,7 +799,7 @@ struct Upsample2x : torch::autograd::Function<Upsample2x> {
 }  // namespace
 
 Tensor group_norm_silu(const Tensor& x, const Tensor& w, const OptT& b_, const OptT& pc_, const OptT& pn_, int64_t groups,
-                       double eps, bool silu) {
+                       double eps, bool silu, bool accum) {
   Tensor b = opt(b_), pc = opt(pc_), pn = opt(pn_);
   const Rows r(x);
   check_channels(w, r.C, "group_norm_silu weight");
@@ -808,18 +809,18 @@ Tensor group_norm_silu(const Tensor& x, const Tensor& w, const OptT& b_, const O
   check_channels(pn, (int64_t)r.N * r.C, "group_norm_silu pre_nc");
   TORCH_CHECK_VALUE(!pn.defined() || (pn.dim() == 2 && pn.size(0) == r.N), "group_norm_silu pre_nc: ", pn.sizes());
   if (any_grad({&x, &w, &b, &pc, &pn}))
-    return GroupNormSilu::apply(wrap(x), wrap(w), wrap(b), wrap(pc), wrap(pn), groups, eps, silu);
+    return GroupNormSilu::apply(wrap(x), wrap(w), wrap(b), wrap(pc), wrap(pn), groups, eps, silu, accum);
   return gn_forward(rows_contig(x), contig16(w), contig16(b), contig16(pc), contig16(pn), groups, eps, silu, Tensor());
 }
 
 // a + b + bias + bias2 (per channel): a block's residual sum with the biases of its last convolutions.
-Tensor add_bias(const Tensor& a, const Tensor& b, const OptT& bias_, const OptT& bias2_) {
+Tensor add_bias(const Tensor& a, const Tensor& b, const OptT& bias_, const OptT& bias2_, bool accum) {
   Tensor bias = opt(bias_), bias2 = opt(bias2_);
   const Rows r(a);
   TORCH_CHECK_VALUE(a.sizes() == b.sizes(), "add_bias: ", a.sizes(), " and ", b.sizes());
   check_channels(bias, r.C, "add_bias bias");
   check_channels(bias2, r.C, "add_bias bias2");
-  if (any_grad({&a, &b, &bias, &bias2})) return AddBias::apply(wrap(a), wrap(b), wrap(bias), wrap(bias2));
+  if (any_grad({&a, &b, &bias, &bias2})) return AddBias::apply(wrap(a), wrap(b), wrap(bias), wrap(bias2), accum);
   return add_bias_forward(rows_contig(a), rows_contig(b), contig16(bias), contig16(bias2));
 }
 
@@ -835,7 +836,7 @@ Tensor upsample2x(const Tensor& x) {
 namespace {
 struct TrainedConv : torch::autograd::Function<TrainedConv> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, std::vector<int64_t> strides,
-                        std::vector<int64_t> padding, std::vector<int64_t> dilation) {
+                        std::vector<int64_t> padding, std::vector<int64_t> dilation, bool accum) {
     Tensor rows = at::empty(w.sizes(), w.options(), at::MemoryFormat::ChannelsLast);
     check(L.eri_conv_weight_order(w.data_ptr(), rows.data_ptr(), (int)w.size(0), (int)w.size(1), (int)(w.size(2) * w.size(3)), 0,
                                   stream()), "conv_weight_order");
@@ -843,6 +844,7 @@ struct TrainedConv : torch::autograd::Function<TrainedConv> {
     ctx->saved_data["s"] = strides;
     ctx->saved_data["p"] = padding;
     ctx->saved_data["d"] = dilation;
+    ctx->saved_data["accum"] = accum;
     return at::conv2d(x, rows, {}, strides, padding, dilation, 1);
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
@@ -852,7 +854,7 @@ struct TrainedConv : torch::autograd::Function<TrainedConv> {
     auto [dx, dw, db] = at::convolution_backward(g[0], x, rows, std::nullopt, ctx->saved_data["s"].toIntVector(),
                                                  ctx->saved_data["p"].toIntVector(), ctx->saved_data["d"].toIntVector(), false,
                                                  std::vector<int64_t>{0, 0}, 1, {nx, nw, false});
-    if (nw && has_grad_buffer(w, at::kBFloat16) && al16(w.grad())) {
+    if (nw && has_grad_buffer(w, at::kBFloat16, ctx->saved_data["accum"].toBool()) && al16(w.grad())) {
       Tensor d = dw.contiguous(at::MemoryFormat::ChannelsLast);
       if (al16(d)) {
         check(L.eri_conv_weight_order(d.data_ptr(), w.grad().data_ptr(), (int)w.size(0), (int)w.size(1),
@@ -860,14 +862,14 @@ struct TrainedConv : torch::autograd::Function<TrainedConv> {
         dw = Tensor();
       }
     }
-    return {dx, dw, Tensor(), Tensor(), Tensor()};
+    return {dx, dw, Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
 }  // namespace
 
 Tensor conv2d_trained(const Tensor& x, const Tensor& w, const std::vector<int64_t>& strides, const std::vector<int64_t>& padding,
-                      const std::vector<int64_t>& dilation) {
-  return TrainedConv::apply(x, w, strides, padding, dilation);
+                      const std::vector<int64_t>& dilation, bool accum) {
+  return TrainedConv::apply(x, w, strides, padding, dilation, accum);
 }
 
 // ------------------------------------------------------------------------------- FLUX single-stream block
@@ -958,11 +960,11 @@ struct SingleStream : torch::autograd::Function<SingleStream> {
     }
     variable_list out(21);
     auto lora = [&](const Tensor& p, const Tensor& at_, const Tensor& bt, bool tr) {
-      if ((flags & kAccumGrad) && has_grad_buffer(p, at::kBFloat16)) return lora_wgrad(at_, bt, p.grad(), tr, true, flags), Tensor();
+      if (has_grad_buffer(p, at::kBFloat16, flags & kAccumGrad)) return lora_wgrad(at_, bt, p.grad(), tr, true, flags), Tensor();
       return lora_wgrad(at_, bt, Tensor(), tr, false, flags);
     };
     auto dense = [&](const Tensor& p, const Tensor& d, const Tensor& xin) {
-      if ((flags & kAccumGrad) && has_grad_buffer(p, at::kBFloat16)) return wgrad(d, xin, p.grad(), flags), Tensor();
+      if (has_grad_buffer(p, at::kBFloat16, flags & kAccumGrad)) return wgrad(d, xin, p.grad(), flags), Tensor();
       return wgrad(d, xin, Tensor(), flags);
     };
     if (need(9)) out[9] = lora(a2, cat, ts2, true);
@@ -985,8 +987,8 @@ struct SingleStream : torch::autograd::Function<SingleStream> {
     if (need(8)) out[8] = lora(bb1, d_h, h1, false);
     if (need(3)) out[3] = dense(w1, d_h, xm2);
     if (need(5)) out[5] = dense(w2, g, cat);
-    if (need(4)) out[4] = col_sum(d_h, b1);
-    if (need(6)) out[6] = col_sum(g, b2);
+    if (need(4)) out[4] = col_sum(d_h, b1, flags & kAccumGrad);
+    if (need(6)) out[6] = col_sum(g, b2, flags & kAccumGrad);
     out[11] = to_bf16(dqs);
     out[12] = to_bf16(dks);
     return out;

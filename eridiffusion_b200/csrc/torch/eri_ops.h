@@ -162,9 +162,9 @@ Tensor lora_wgrad(const Tensor& a_tok, const Tensor& b_tok, Tensor out, bool tra
 Tensor lora_transposed(const Tensor& m);
 Tensor gate_rows(const Tensor& x, const Tensor& y2, const Tensor& gate, int64_t rows_per_batch);
 bool lora_rank_ok(int64_t r);
-// Adds `g` into p.grad in place when p has one of that type (the arena views), and returns an undefined tensor
-// then; otherwise returns the gradient for autograd to store.
-bool has_grad_buffer(const Tensor& p, at::ScalarType t);
+// Whether p's gradient may be added into p.grad in place (the arena views) instead of being returned for autograd to
+// store. ``allowed``: the caller's switch (kAccumGrad).
+bool has_grad_buffer(const Tensor& p, at::ScalarType t, bool allowed);
 
 OptT linear(const Tensor& x, const Tensor& w, const OptT& bias, const OptT& la, const OptT& lb, double scale, int act,
             const OptT& residual, const OptT& gate, const OptT& wt, int flags);
@@ -172,16 +172,16 @@ std::vector<Tensor> linear_pair(const std::vector<OptT>& s0, double sc0, const s
                                 bool emit_pre, int act_in, int flags);
 Tensor linear_glu(const Tensor& x, const Tensor& w, const OptT& bias, const OptT& la, const OptT& lb, double scale,
                   int code, const OptT& wt, int flags);
-Tensor small_linear(const Tensor& x, const Tensor& w, const OptT& bias, bool silu_in);
+Tensor small_linear(const Tensor& x, const Tensor& w, const OptT& bias, bool silu_in, bool accum);
 Tensor small_wgrad(const Tensor& dy2, const Tensor& xin, double scale, const Tensor& accum);
 Tensor small_dgrad(const Tensor& dy2, const Tensor& w);
 int prepare_lora_transposes(const std::vector<Tensor>& mats);
-Tensor col_sum(const Tensor& x2, const Tensor& p);
+Tensor col_sum(const Tensor& x2, const Tensor& p, bool accum);
 void invalidate_lora_transposes(const std::vector<Tensor>& mats);
 
 // ---- block_ops.cpp
 std::vector<Tensor> norm_modulate(const Tensor& x, const OptT& scale, const OptT& shift, const OptT& weight,
-                                  const OptT& bias, double eps, bool rms, bool skip);
+                                  const OptT& bias, double eps, bool rms, bool skip, bool accum);
 std::vector<Tensor> qknorm_rope_joint(const std::vector<OptT>& flat, const OptT& cos, const OptT& sin, int64_t heads,
                                       double eps);
 Tensor gate_residual(const OptT& x, const Tensor& y, const OptT& gate);
@@ -197,11 +197,11 @@ Tensor attention_qkv_rope(const Tensor& qkv, const Tensor& wq, const Tensor& wk,
                           int64_t heads, double eps);
 Tensor mse_loss(const Tensor& pred, const Tensor& target, const OptT& weight);
 Tensor group_norm_silu(const Tensor& x, const Tensor& weight, const OptT& bias, const OptT& pre_c, const OptT& pre_nc,
-                       int64_t groups, double eps, bool silu);
-Tensor add_bias(const Tensor& a, const Tensor& b, const OptT& bias, const OptT& bias2);
+                       int64_t groups, double eps, bool silu, bool accum);
+Tensor add_bias(const Tensor& a, const Tensor& b, const OptT& bias, const OptT& bias2, bool accum);
 Tensor upsample2x(const Tensor& x);
 Tensor conv2d_trained(const Tensor& x, const Tensor& w, const std::vector<int64_t>& stride, const std::vector<int64_t>& padding,
-                      const std::vector<int64_t>& dilation);
+                      const std::vector<int64_t>& dilation, bool accum);
 Tensor single_stream(const Tensor& xm, const Tensor& x, const Tensor& gate, const Tensor& w1, const OptT& b1,
                      const Tensor& w2, const OptT& b2, const OptT& a1, const OptT& bb1, double s1, const OptT& a2,
                      const OptT& bb2, double s2, const OptT& qs, const OptT& ks, const OptT& cos, const OptT& sin,

@@ -92,8 +92,8 @@ Tensor undef() { return Tensor(); }
 
 bool gemm_supported(int64_t M, int64_t N, int64_t K) { return M >= 128 && N >= 16 && K >= 8 && K % 8 == 0 && N % 8 == 0; }
 bool lora_rank_ok(int64_t r) { return r == 16 || r == 32 || r == 64; }
-bool has_grad_buffer(const Tensor& p, at::ScalarType t) {
-  if (!p.is_leaf() || !p.requires_grad()) return false;
+bool has_grad_buffer(const Tensor& p, at::ScalarType t, bool allowed) {
+  if (!allowed || !p.is_leaf() || !p.requires_grad()) return false;
   // torch.autograd.grad and backward(inputs=...) want the gradient itself, and so does whoever hooked the parameter
   const auto* asked = torch::autograd::get_current_graph_task_exec_info();
   if (asked && !asked->empty()) return false;
@@ -330,8 +330,8 @@ Tensor lora_transposed(const Tensor& m) {
 
 // Column sums of x2 [M, N] for the parameter p (a bias): added straight into p.grad when it has a buffer of that
 // type (an undefined tensor is returned then), else returned.
-Tensor col_sum(const Tensor& x2, const Tensor& p) {
-  const bool acc = has_grad_buffer(p, x2.scalar_type());
+Tensor col_sum(const Tensor& x2, const Tensor& p, bool accum) {
+  const bool acc = has_grad_buffer(p, x2.scalar_type(), accum);
   if (x2.size(0) > 0 && rows_ok(x2) && x2.size(1) % 8 == 0 && (!acc || al16(p.grad()))) {
     Tensor out = acc ? p.grad() : empty_bf16({x2.size(1)}, x2);
     check(L.eri_col_sum(x2.data_ptr(), x2.stride(0), out.data_ptr(), (int)x2.size(0), (int)x2.size(1), acc, stream()),
@@ -402,20 +402,20 @@ LinGrads linear_grads(const Tensor& dy2, const Tensor& x2, const Tensor& w, cons
     g.dx = g.dx.view(shp);
   }
   if (nw) {
-    if ((flags & kAccumGrad) && has_grad_buffer(w, x2.scalar_type()))
+    if (has_grad_buffer(w, x2.scalar_type(), flags & kAccumGrad))
       wgrad(dy2, x2, w.grad(), flags);       // beta = 1 into the (arena) gradient view
     else
       g.dw = wgrad(dy2, x2, Tensor(), flags);
   }
-  if (nb) g.db = col_sum(dy2, bias);
+  if (nb) g.db = col_sum(dy2, bias, flags & kAccumGrad);
   if (r && na) {
-    if ((flags & kAccumGrad) && has_grad_buffer(la, x2.scalar_type()))
+    if (has_grad_buffer(la, x2.scalar_type(), flags & kAccumGrad))
       lora_wgrad(x2, ts, la.grad(), true, true, flags);
     else
       g.da = lora_wgrad(x2, ts, Tensor(), true, false, flags);
   }
   if (r && nlb) {
-    if ((flags & kAccumGrad) && has_grad_buffer(lb, h.scalar_type()))
+    if (has_grad_buffer(lb, h.scalar_type(), flags & kAccumGrad))
       lora_wgrad(dy2, h, lb.grad(), false, true, flags);
     else
       g.dlb = lora_wgrad(dy2, h, Tensor(), false, false, flags);
@@ -701,20 +701,20 @@ struct FusedLinearPair : torch::autograd::Function<FusedLinearPair> {
       const Tensor *t = &sv[9 * i], &x2 = t[0], &w = t[1], &la = t[3], &lb = t[4], &h = t[5];
       Tensor* g = &out[i * Stream::kCount];
       if (need(i, Stream::w)) {
-        if ((flags & kAccumGrad) && has_grad_buffer(w, x2.scalar_type()))
+        if (has_grad_buffer(w, x2.scalar_type(), flags & kAccumGrad))
           wgrad(dy2[i], x2, w.grad(), flags);
         else
           g[Stream::w] = wgrad(dy2[i], x2, Tensor(), flags);
       }
-      if (need(i, Stream::b)) g[Stream::b] = col_sum(dy2[i], t[2]);
+      if (need(i, Stream::b)) g[Stream::b] = col_sum(dy2[i], t[2], flags & kAccumGrad);
       if (need(i, Stream::la)) {
-        if ((flags & kAccumGrad) && has_grad_buffer(la, x2.scalar_type()))
+        if (has_grad_buffer(la, x2.scalar_type(), flags & kAccumGrad))
           lora_wgrad(x2, ts[i], la.grad(), true, true, flags);
         else
           g[Stream::la] = lora_wgrad(x2, ts[i], Tensor(), true, false, flags);
       }
       if (need(i, Stream::lb)) {
-        if ((flags & kAccumGrad) && has_grad_buffer(lb, h.scalar_type()))
+        if (has_grad_buffer(lb, h.scalar_type(), flags & kAccumGrad))
           lora_wgrad(dy2[i], h, lb.grad(), false, true, flags);
         else
           g[Stream::lb] = lora_wgrad(dy2[i], h, Tensor(), false, false, flags);
@@ -850,13 +850,13 @@ Tensor small_forward(const Tensor& x, const Tensor& w, const Tensor& bias, bool 
 }
 
 struct SmallLinear : torch::autograd::Function<SmallLinear> {
-  static Tensor forward(AutogradContext* ctx, const OptT& x_o, const OptT& w_o, const OptT& bias_o, bool silu_in) {
+  static Tensor forward(AutogradContext* ctx, const OptT& x_o, const OptT& w_o, const OptT& bias_o, bool silu_in, bool accum) {
     const Tensor x = opt(x_o), w = opt(w_o), bias = opt(bias_o);
     if (ctx) ctx->saved_data["args"] = Args({&x, &w, &bias}).mask;
     Tensor x2;
     Tensor y = small_forward(x, w, bias, silu_in, &x2);
     ctx->save_for_backward({x2, w, bias});
-    ctx->saved_data["m"] = std::vector<int64_t>{silu_in};
+    ctx->saved_data["m"] = std::vector<int64_t>{silu_in, accum};
     ctx->saved_data["shp"] = x.sizes().vec();
     return y;
   }
@@ -864,7 +864,8 @@ struct SmallLinear : torch::autograd::Function<SmallLinear> {
     auto sv = ctx->get_saved_variables();
     const Tensor &x2 = sv[0], &w = sv[1];
     const Args args(ctx->saved_data["args"].toInt());
-    const bool silu_in = ctx->saved_data["m"].toIntVector()[0];
+    const auto m = ctx->saved_data["m"].toIntVector();
+    const bool silu_in = m[0];
     const Tensor& dy = gout[0];
     Tensor dy2 = dy.reshape({-1, dy.size(-1)});
     if (dy2.stride(1) != 1) dy2 = dy2.contiguous();
@@ -879,21 +880,21 @@ struct SmallLinear : torch::autograd::Function<SmallLinear> {
       Tensor xin = silu_in ? at::silu(x2) : x2;
       if (!native || !rows_ok(xin))
         dw = at::mm(dy2.t(), xin);
-      else if (has_grad_buffer(w, at::kBFloat16) && al16(w.grad()))
+      else if (has_grad_buffer(w, at::kBFloat16, m[1]) && al16(w.grad()))
         small_wgrad(dy2, xin, 1.0, w.grad());      // added into the (arena) gradient view
       else
         dw = small_wgrad(dy2, xin, 1.0, Tensor());
     }
     if (args.need(ctx, 2)) db = dy2.sum(0);
-    return {dx, dw, db, Tensor()};
+    return {dx, dw, db, Tensor(), Tensor()};
   }
 };
 
 }  // namespace
 
-Tensor small_linear(const Tensor& x, const Tensor& w, const OptT& bias_, bool silu_in) {
+Tensor small_linear(const Tensor& x, const Tensor& w, const OptT& bias_, bool silu_in, bool accum) {
   Tensor bias = opt(bias_);
-  if (any_grad({&x, &w, &bias})) return SmallLinear::apply(wrap(x), wrap(w), wrap(bias), silu_in);
+  if (any_grad({&x, &w, &bias})) return SmallLinear::apply(wrap(x), wrap(w), wrap(bias), silu_in, accum);
   return small_forward(x, w, bias, silu_in, nullptr);
 }
 

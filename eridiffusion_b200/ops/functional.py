@@ -88,7 +88,7 @@ def norm_modulate_skip(x, scale=None, shift=None, weight=None, bias=None, eps=1e
     native path the gradients of both branches are summed inside the norm's backward kernel."""
     if _NORM_SKIP and _native_ok(x, scale, shift, weight, bias) and x.dim() == 3 and x.shape[-1] % 8 == 0 \
             and torch.is_grad_enabled() and x.requires_grad:
-        return N.ops().norm_modulate(x, scale, shift, weight, bias, eps, rms, True)
+        return N.ops().norm_modulate(x, scale, shift, weight, bias, eps, rms, True, _ACCUM_INTO_GRAD)
     return norm_modulate(x, scale, shift, weight, bias, eps, rms), x
 
 
@@ -99,7 +99,7 @@ _NORM_SKIP = os.environ.get("ERI_B200_NORM_SKIP", "0") == "1"
 def norm_modulate(x, scale=None, shift=None, weight=None, bias=None, eps=1e-6, rms=False):
     if _native_ok(x, scale, shift, weight, bias) and x.dim() == 3 and x.shape[-1] % 8 == 0 \
             and x.shape[-1] <= 8192:
-        return N.ops().norm_modulate(x, scale, shift, weight, bias, eps, rms, False)[0]
+        return N.ops().norm_modulate(x, scale, shift, weight, bias, eps, rms, False, _ACCUM_INTO_GRAD)[0]
     return R.norm_modulate(x, scale, shift, weight, bias, eps, rms)
 
 
@@ -590,7 +590,7 @@ def small_linear(x, w, bias=None, silu_in=False):
     """Linear on a handful of rows (adaLN modulation and embedders); SiLU on the input optional."""
     rows = x.numel() // x.shape[-1]
     if _native_ok(x, w, bias) and rows <= 8 and x.shape[-1] % 8 == 0 and x.shape[-1] * rows <= 50000:
-        return N.ops().small_linear(x, w, bias, silu_in)
+        return N.ops().small_linear(x, w, bias, silu_in, _ACCUM_INTO_GRAD)
     xin = torch.nn.functional.silu(x) if silu_in else x
     return torch.nn.functional.linear(xin, w, bias)
 
@@ -778,7 +778,7 @@ def group_norm_silu(x, weight, bias=None, groups=32, eps=1e-5, silu=True, pre_c=
     bias of the convolution that produced x and a per-sample embedding), in the same pass on the native path."""
     C = x.shape[1] if x.dim() == 4 else x.shape[-1]
     if _native_ok(x, weight, bias, pre_c, pre_nc) and C % 8 == 0 and C % groups == 0 and C <= 8192 and groups <= 4096:
-        return N.ops().group_norm_silu(x, weight, bias, pre_c, pre_nc, groups, eps, silu)
+        return N.ops().group_norm_silu(x, weight, bias, pre_c, pre_nc, groups, eps, silu, _ACCUM_INTO_GRAD)
     nchw = x.dim() == 4
     if nchw:
         Nn, C, H, W = x.shape
@@ -803,7 +803,7 @@ def add_bias(a, b, bias=None, bias2=None):
     convolutions. [N, HW, C] or channels-last [N, C, H, W]."""
     C = a.shape[1] if a.dim() == 4 else a.shape[-1]
     if _native_ok(a, b, bias, bias2) and C % 8 == 0 and a.shape == b.shape:
-        return N.ops().add_bias(a, b, bias, bias2)
+        return N.ops().add_bias(a, b, bias, bias2, _ACCUM_INTO_GRAD)
     y = a + b
     for t in (bias, bias2):
         if t is not None:
@@ -844,7 +844,7 @@ def conv_no_bias(conv, x):
             and w.is_contiguous() and w.shape[1] % 8 == 0 and w.shape[0] <= 65535 and 1 < w.shape[2] * w.shape[3] <= 25 \
             and w.data_ptr() % 16 == 0:
         # (a parameter of the flat arena; a weight already in channels-last order needs no copy)
-        return N.ops().conv2d_trained(x, w, list(conv.stride), list(conv.padding), list(conv.dilation))
+        return N.ops().conv2d_trained(x, w, list(conv.stride), list(conv.padding), list(conv.dilation), _ACCUM_INTO_GRAD)
     return torch.nn.functional.conv2d(x, w, None, conv.stride, conv.padding, conv.dilation, conv.groups)
 
 
