@@ -102,9 +102,11 @@ struct Lib {
 extern Lib L;
 extern std::atomic<long long> g_launches;
 
-// Switches of ops/functional.py that the nodes honour, read there at every call.
-enum Flag : int { kPdl = 1, kRankStream = 2, kPair = 4, kGroup = 8, kActEpilogue = 16, kWgrad = 32, kAccumGrad = 64,
+// Switches and rules of ops/functional.py that the nodes honour, evaluated there at every call. From kFewTilesShift up: the
+// most 256 x 256 tiles that a product may have and still run on the one-CTA kernel.
+enum Flag : int { kPdl = 1, kRankStream = 2, kPair = 4, kGroup = 8, kActOutside = 16, kWgrad = 32, kAccumGrad = 64,
                   kNativeGemm = 128 };
+constexpr int kFewTilesShift = 8;
 
 inline void check(int code, const char* what) {
   g_launches.fetch_add(1, std::memory_order_relaxed);

@@ -14,14 +14,6 @@ namespace eri_ops {
 
 namespace {
 
-int few_tile_limit() {
-  static const int v = [] {
-    const char* e = getenv("ERI_B200_PAIR_MIN_TILES");
-    return e ? atoi(e) : 36;
-  }();
-  return v;
-}
-
 struct Built {
   EriGemmArgs g;
   Tensor out;
@@ -72,7 +64,7 @@ void launch(const EriGemmArgs& g, int flags) {
   // Few pair tiles (the 512-token text stream against a 3072-wide weight: 24 tiles for 74 CTA pairs) leave
   // most SMs idle; the one-CTA kernel's 128-column tiles spread the same work over four times as many CTAs.
   const bool few = !(g.a_mn || g.glu) &&
-                   (int64_t)((g.M + 255) / 256) * ((g.N + 255) / 256) <= few_tile_limit();
+                   (int64_t)((g.M + 255) / 256) * ((g.N + 255) / 256) <= (flags >> kFewTilesShift);
   if (((flags & kPair) || g.a_mn || g.glu) && g.M >= 256 && g.N >= 256 && !few) {
     const int code = L.eri_gemm2_bf16(&g, stream());
     if (code != -30) return check(code, "gemm2_bf16");
@@ -80,10 +72,6 @@ void launch(const EriGemmArgs& g, int flags) {
   TORCH_CHECK(!(g.a_mn || g.glu), "gemm: a_mn / glu need the two-CTA kernel's shape range (M=", g.M, ", N=", g.N,
               ", K=", g.K, ")");
   check(L.eri_gemm_bf16(&g, stream()), "gemm_bf16");
-}
-
-bool act_outside_epilogue(int64_t M, int64_t N, int64_t K, int flags) {
-  return !(flags & kActEpilogue) && K <= 4096 && M * N >= (1 << 25);
 }
 
 Tensor undef() { return Tensor(); }
@@ -456,7 +444,7 @@ LinOut linear_forward(const Tensor& x, const Tensor& w, const Tensor& bias, cons
     o.bias = bias;
     o.pdl = flags & kPdl;
     if (act && keep) r.pre = empty_bf16({M, N}, x);
-    const bool split = r.pre.defined() && !res2.defined() && !r.gate.defined() && act_outside_epilogue(M, N, K, flags);
+    const bool split = r.pre.defined() && !res2.defined() && !r.gate.defined() && (flags & kActOutside);
     if (split) {
       // training keeps the pre-activation anyway: the GEMM writes it as its output and the activation is a pass
       // of its own (cheaper than storing both from the epilogue)
@@ -601,7 +589,7 @@ struct FusedLinearPair : torch::autograd::Function<FusedLinearPair> {
     }
     // Training keeps the pre-activation anyway: the GEMM then writes it as its output and the activation is a
     // pass of its own (storing both from the epilogue costs the GEMM more than that pass does).
-    bool unfuse = act && act_outside_epilogue(M[0], N[0], K[0], (int)flags);
+    bool unfuse = act && (flags & kActOutside);
     for (int i = 0; i < 2; ++i) unfuse = unfuse && pre[i].defined() && !o[i].residual.defined() && !gv[i].defined();
     for (int i = 0; i < 2; ++i) {
       if (unfuse) {

@@ -446,11 +446,13 @@ def lora_wgrad(a_tok, b_tok, out=None, transpose_out=False, accumulate=False):
 _ACCUM_INTO_GRAD = os.environ.get("ERI_B200_ACCUM_INTO_GRAD", "1") == "1"
 
 
-def _flags() -> int:
-    """The switches of this module that the native nodes honour (``Flag`` in csrc/torch/eri_ops.h)."""
+def _flags(x=None, w=None, act=None) -> int:
+    """The switches of this module that the native nodes honour (``Flag`` in csrc/torch/eri_ops.h), with the rule for the
+    activation of a linear ``act(x w^T)``."""
+    outside = act is not None and x.shape[-1] > 0 and _act_outside_epilogue(x.numel() // x.shape[-1], w.shape[0], x.shape[-1])
     return ((1 if _pdl_ok() else 0) | (2 if _RANK_STREAM else 0) | (4 if _GEMM_PAIR else 0) | (8 if _GEMM_GROUP else 0)
-            | (16 if _ACT_EPILOGUE else 0) | (32 if _WGRAD_NATIVE else 0) | (64 if _ACCUM_INTO_GRAD else 0)
-            | (128 if _GEMM_NATIVE == "native" else 0))
+            | (16 if outside else 0) | (32 if _WGRAD_NATIVE else 0) | (64 if _ACCUM_INTO_GRAD else 0)
+            | (128 if _GEMM_NATIVE == "native" else 0) | (max(0, min(_PAIR_MIN_TILES, 1 << 20)) << 8))
 
 
 def prepare_lora_transposes(matrices):
@@ -481,7 +483,7 @@ def linear(x, w, bias=None, lora=None, act=None, residual=None, gate=None, wt=No
     cached transpose of a frozen W ([K, N]) that lets the input-gradient GEMM read a K-major operand."""
     if _BACKEND == "fused" and x.is_cuda:
         a, b, s = lora if lora is not None else (None, None, 1.0)
-        y = N.ops().linear(x, w, bias, a, b, s, _ACT_CODE[act], residual, gate, wt, _flags())
+        y = N.ops().linear(x, w, bias, a, b, s, _ACT_CODE[act], residual, gate, wt, _flags(x, w, act))
         if y is not None:
             return y
     y = R.linear(x, w, bias, lora, act, None, None)
@@ -520,7 +522,8 @@ def linear_pair(x0, lin0, x1, lin1, act=None, emit_pre=False, act_in=None, x_pre
         a0, bb0, s0 = lo0 if lo0 is not None else (None, None, 1.0)
         a1, bb1, s1 = lo1 if lo1 is not None else (None, None, 1.0)
         return tuple(N.ops().linear_pair([x0, x_pre[0], w0, b0, a0, bb0, *rg0], s0, [x1, x_pre[1], w1, b1, a1, bb1, *rg1],
-                                         s1, _ACT_CODE[act], emit_pre, _ACT_CODE[act_in], _flags()))
+                                         s1, _ACT_CODE[act], emit_pre, _ACT_CODE[act_in],
+                                         _flags(x0, w0, act)))
 
     if emit_pre or act_in is not None:
         return apply((r0, g0), (r1, g1))
