@@ -470,37 +470,6 @@ __global__ void gate_residual_kernel(const bf16* __restrict__ x, const bf16* __r
     reinterpret_cast<bf16x8*>(out)[i] = pack8(c);
   }
 }
-// d_gate[b, d] += sum over the batch's tokens of dout * y
-__global__ void gate_grad_kernel(const bf16* __restrict__ dout, const bf16* __restrict__ y,
-                                 float* __restrict__ dgate, int rows, int D, int rows_per_batch,
-                                 int rows_per_cta) {
-  const int nvec = D >> 3;
-  const int row0 = blockIdx.x * rows_per_cta, row1 = min(rows, row0 + rows_per_cta);
-  for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
-    float acc[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-    int cur_b = row0 / rows_per_batch;
-    for (int row = row0; row < row1; ++row) {
-      int b = row / rows_per_batch;
-      if (b != cur_b) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          atomicAdd(dgate + (size_t)cur_b * D + v * 8 + j, acc[j]);
-          acc[j] = 0.f;
-        }
-        cur_b = b;
-      }
-      float a[8], c[8];
-      unpack8(reinterpret_cast<const bf16x8*>(dout + (size_t)row * D)[v], a);
-      unpack8(reinterpret_cast<const bf16x8*>(y + (size_t)row * D)[v], c);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] += a[j] * c[j];
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) atomicAdd(dgate + (size_t)cur_b * D + v * 8 + j, acc[j]);
-  }
-}
 
 // ------------------------------------------------------------------ activations
 // mode 0 GELU(tanh), 1 SiLU. bwd: dx = dy * f'(x)
@@ -861,15 +830,6 @@ int eri_gate_residual(const void* x, const void* y, const void* gate, void* out,
   gate_residual_kernel<<<stream_grid(nvec, 256), 256, 0, (cudaStream_t)stream>>>(
       (const bf16*)x, (const bf16*)y, (const bf16*)gate, (bf16*)out, nvec, D, rows_per_batch,
       mod_stride);
-  ERI_LAUNCH_CHECK();
-}
-
-int eri_gate_grad(const void* dout, const void* y, float* dgate, int rows, int D,
-                  int rows_per_batch, void* stream) {
-  if (D % 8 != 0) return -1;
-  const int rpc = 32;
-  gate_grad_kernel<<<(rows + rpc - 1) / rpc, 256, 0, (cudaStream_t)stream>>>(
-      (const bf16*)dout, (const bf16*)y, dgate, rows, D, rows_per_batch, rpc);
   ERI_LAUNCH_CHECK();
 }
 

@@ -3,8 +3,9 @@
 //
 // What bounds it: a training step at a few hundred tokens is a chain of launches of 3-20 us each, and the
 // same nodes written in Python (an autograd.Function, a ctypes call with one setattr per argument) took
-// 20-30 us of host time per launch. Here a launch costs 2-4 us and the backward runs without the
-// interpreter lock.
+// 20-30 us of host time per launch. Inside a node a launch costs 2-4 us here and the backward runs without the
+// interpreter lock; the Python of a model between its nodes is not in that figure (a whole training pass of a small
+// model comes to 12 us per launch).
 #pragma once
 #include <torch/extension.h>
 #include <c10/cuda/CUDAStream.h>
@@ -42,7 +43,6 @@ using torch::autograd::variable_list;
                           const float*, const float*, void*, float*, float*, int, int, int, int, int, int,       \
                           float, int, int, int, void*))                                                          \
   X(eri_gate_residual, (const void*, const void*, const void*, void*, long long, int, int, int, void*))          \
-  X(eri_gate_grad, (const void*, const void*, float*, int, int, int, void*))                                     \
   X(eri_act_fwd, (const void*, void*, long long, int, void*))                                                    \
   X(eri_act_bwd, (const void*, const void*, void*, long long, int, void*))                                       \
   X(eri_act_fwd_rows, (const void*, long long, void*, long long, int, int, int, void*))                          \

@@ -84,7 +84,6 @@ _SIGNATURES = {
     "eri_qknorm_rope_bwd": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F,
                             _I, _I, _I, _P],
     "eri_gate_residual": [_P, _P, _P, _P, _L, _I, _I, _I, _P],
-    "eri_gate_grad": [_P, _P, _P, _I, _I, _I, _P],
     "eri_slot_reduce": [_P, _P, _I, _L, _F, _I, _P],
     "eri_act_fwd": [_P, _P, _L, _I, _P],
     "eri_act_bwd": [_P, _P, _P, _L, _I, _P],
