@@ -7,7 +7,7 @@
 // 1.25 GB. A CTA holds a whole token in registers (the sums need a block reduction, nothing is read twice), and
 // q, k are read inside the projection's output and their gradients written inside its gradient.
 // As separate fp32 passes (contiguous copies, norm, two multiplies, add, stack, cast per operand and direction) the
-// same work took 7.2 ms of a 46 ms training pass over one block at 19008 tokens; the pass now takes 40.2 ms.
+// same work took 7.2 ms of a 47 ms training pass over one block at 19008 tokens; the pass with this kernel takes 41-42 ms.
 // Reference: src/models/ltx2_model.rs:180-260 (QK-norm across heads, rotary over the inner dimension).
 #include "ptx.cuh"
 
