@@ -2,7 +2,8 @@
 the device, a handful of launches), one per hot kernel:
 
     python -m eridiffusion_b200.cli.profile_target gemm|gemm_lora|rank_stream|attn_fwd|attn_bwd|norm|qknorm|adamw|gemv|
-        elementwise|groupnorm|token_route|dequant|attn_masked|small_linear_bwd|slot_reduce|gemm_small_m|gemm_group
+        elementwise|groupnorm|token_route|dequant|attn_masked|small_linear_bwd|slot_reduce|gemm_small_m|gemm_group|
+        gemm_few|attn_wide|attn_bias|norm_rope|norm_rows|column_sums|conv_layout|conv_companions|ema
 
 Meant to be run as ``ncu --set full --clock-control none -k regex:<kernel> -s 2 -c 1 ... python -m
 eridiffusion_b200.cli.profile_target <what>`` after the same command line exited 0 without ncu.
@@ -171,6 +172,65 @@ def main():
             F.gemm_native(**kws[0])
             F.gemm_native(**kws[1])
         assert F.gemm_error_check() == 0
+    elif what == "gemm_few":
+        # a T5-style down-projection of one 256-token caption; four weights of 84 MB, so that each launch reads DRAM
+        a, ws = r(256, 10240), [r(4096, 10240) for _ in range(4)]
+        for w in ws:
+            F.gemm_native(a, w)
+        assert F.gemm_error_check() == 0
+    elif what == "attn_wide":
+        # spatial attention in the middle of an image autoencoder at 1024 x 1024: 16384 tokens, one head of 512
+        q, k, v = r(1, 16384, 3, 1, 512).unbind(2)
+        for _ in range(iters):
+            F.attention(q, k, v)
+        assert F.kernel_error_check() == {}
+    elif what == "attn_bias":
+        # T5-style attention of one 256-token caption with its relative-position bias
+        q, k, v = r(1, 256, 3, 64, 64).unbind(2)
+        bias = r(1, 64, 256, 256)
+        for _ in range(iters):
+            F.attention(q, k, v, scale=1.0, mask=bias)
+        assert F.kernel_error_check() == {}
+    elif what == "norm_rope":
+        # QK-norm over the whole width + rotary embedding of a video block, 9504 tokens x 4096, inside its attention
+        qkv = r(1, 9504, 3 * 4096).requires_grad_()
+        w, (cos, sin) = r(4096), (torch.rand(9504, 2048, device=dev) for _ in "cs")
+        for _ in range(2):
+            F.attention_qkv_rope(qkv, w, w, cos, sin, 32).backward(r(1, 9504, 4096))
+    elif what == "norm_rows":
+        # the text rows of a video block: a CTA per row
+        x, mod = r(1, 256, 4096).requires_grad_(), r(1, 2 * 4096)
+        sc, sh = mod.split(4096, -1)
+        for _ in range(iters):
+            F.norm_modulate(x, sc, sh).backward(torch.ones_like(x))
+        assert F.kernel_error_check() == {}
+    elif what == "column_sums":
+        # gradients of a bias, of norm parameters and of a gate over [4096, 12288] / [4096, 3072] rows
+        x, b, w = r(1, 4096, 256), r(12288).requires_grad_(), r(12288, 256)
+        y, nw, nb, gate = r(1, 4096, 3072), r(3072).requires_grad_(), r(3072).requires_grad_(), r(1, 3072).requires_grad_()
+        for _ in range(iters):
+            F.linear(x, w, b).backward(r(1, 4096, 12288))
+            F.norm_modulate(y, weight=nw, bias=nb).backward(y)
+            F.gate_residual(None, y, gate).backward(y)
+    elif what == "conv_layout":
+        # weight of a trained 1280-channel 3x3 convolution: to channels-last order, gradient added back in parameter order
+        convs = [torch.nn.Conv2d(1280, 1280, 3, padding=1, device=dev, dtype=torch.bfloat16) for _ in range(4)]
+        x = r(1, 1280, 16, 16).contiguous(memory_format=torch.channels_last)
+        for c in convs:
+            c.weight.grad = torch.zeros_like(c.weight)
+            F.conv_no_bias(c, x).backward(x)
+    elif what == "conv_companions":
+        # residual sum with a bias, and upsampling, at the decoder's largest level
+        x = r(1, 256, 512, 512).contiguous(memory_format=torch.channels_last)
+        b = r(256)
+        for _ in range(iters):
+            F.add_bias(x, x, b)
+            F.upsample2x(x)
+    elif what == "ema":
+        from ..optim import EMA, ParamArena
+        avg = EMA(ParamArena([torch.nn.Parameter(r(112_000_000))]), 0.999)
+        for _ in range(iters):
+            avg.update()
     else:
         raise SystemExit(f"unknown target {what}")
     torch.cuda.synchronize()
