@@ -50,7 +50,7 @@ def test_bias_attention(B, Lq, Lk, H, D, shape):
     assert F.ATTENTION_CALLS["native"] == calls + 1 and FA.check_error() == 0
     if key_only:                         # a mask of keys alone keeps its own kernel (bf16 probabilities)
         return
-    # fp32 throughout (probabilities as two bf16 terms): what is left is one rounding of the result to bf16, 2^-9
+    # fp32 throughout (probabilities as three bf16 terms): what is left is one rounding of the result to bf16, 2^-9
     assert ((o.double() - r).norm() / r.norm()).item() < 2 ** -8.5
     e0, e1 = ((t.double() - r).norm().item() for t in (lib, o))
     assert e1 <= e0 * 1.02

@@ -1,12 +1,16 @@
 """Residual blocks of the UNet and the autoencoder with their biases folded into the ops around the convolutions: the same
 values and gradients as the plain sequence, and every hook or replaced module is still called."""
+import copy
+
 import pytest
 import torch
 import torch.nn as nn
 
+from eridiffusion_b200.models.layers import channels_last_convs
 from eridiffusion_b200.models.sdxl_unet import ResBlock, SDXLConfig
-from eridiffusion_b200.models.vae import _Res
+from eridiffusion_b200.models.vae import Encoder, VaeConfig, _Res, _run
 from eridiffusion_b200.ops import functional as F
+from eridiffusion_b200.optim import ParamArena
 
 pytestmark = pytest.mark.gpu
 KW = dict(device="cuda", dtype=torch.bfloat16)
@@ -76,3 +80,81 @@ def test_hooks_of_an_autoencoder_block_fire(name):
     getattr(blk, name).register_full_backward_hook(lambda *a: seen.append(a) and None)
     blk(nhwc(2, 64, 8, 8).requires_grad_()).sum().backward()
     assert len(seen) == 1
+
+
+def gradients(m, call, dy):
+    """Output, input gradients and every parameter's gradient of ``call(m)`` -> (output, inputs)."""
+    for p in m.parameters():
+        p.grad = None if p.grad is None else p.grad.zero_()
+    y, ins = call(m)
+    y.backward(dy.to(y.dtype))
+    return {"out": y.detach(), **{f"in{i}": t.grad for i, t in enumerate(ins)}, **{n: p.grad for n, p in m.named_parameters()}}
+
+
+def no_further_than_plain_bf16(m, call, arena):
+    """The folded form, the plain bf16 sequence and fp32 on the same weights. Both bf16 forms round every activation and
+    gradient (2^-9 each), in another order: their errors are two draws of the same size, of which one may be up to three
+    times the other. A bias dropped, added twice or without its gradient is off by its own size, some hundred times that."""
+    torch.manual_seed(0)
+    ref, plain = copy.deepcopy(m).float(), copy.deepcopy(m)
+    if arena == "arena":
+        ParamArena(list(m.parameters()))
+    else:
+        channels_last_convs(m)
+    dy = None
+    F.set_backend("eager")
+    try:
+        dy = torch.randn_like(call(ref)[0])
+        want, lib = gradients(ref, call, dy), gradients(plain, call, dy)
+    finally:
+        F.set_backend("fused")
+    got = gradients(m, call, dy)
+    assert got.keys() == want.keys()
+    for k, w in want.items():
+        assert got[k] is not None, k
+        e, e0 = (((t[k].double() - w.double()).norm() / w.double().norm()).item() for t in (got, lib))
+        assert e <= 3 * e0 + 2.0 ** -8, (k, e, e0)
+
+
+def on_input(x, f):
+    def call(m):
+        p = next(m.parameters())
+        ins = [t.to(p.dtype).detach().requires_grad_() for t in x]
+        return f(m, *ins), ins
+    return call
+
+
+@pytest.mark.parametrize("arena", ["arena", "channels last"])
+@pytest.mark.parametrize("cin,cout", [(64, 64), (64, 128)])
+def test_unet_block(cin, cout, arena):
+    m = randomised(ResBlock(cin, cout, 128, SDXLConfig(), torch.bfloat16, "cuda"))
+    no_further_than_plain_bf16(m, on_input([nhwc(2, cin, 12, 10), torch.randn(2, 128, **KW)], lambda m, x, e: m(x, e)), arena)
+
+
+class ConvThenBlock(nn.Module):
+    def __init__(self, cin, cout):
+        super().__init__()
+        self.conv, self.blk = nn.Conv2d(32, cin, 3, padding=1, **KW), _Res(cin, cout, 32, KW)
+
+
+@pytest.mark.parametrize("arena", ["arena", "channels last"])
+@pytest.mark.parametrize("deferred", [False, True])
+@pytest.mark.parametrize("cin,cout", [(64, 64), (64, 128)])
+def test_autoencoder_block(cin, cout, deferred, arena):
+    """``deferred``: the bias of the convolution in front is added by the block."""
+    m = randomised(ConvThenBlock(cin, cout))
+    seen = []
+
+    def call(m, x):
+        if not deferred:
+            return m.blk(m.conv(x))
+        seen.append(m.blk.fusable(x))
+        return _run([m.conv, m.blk], x, lambda t: t)
+    no_further_than_plain_bf16(m, on_input([nhwc(2, 32, 12, 10)], call), arena)
+    assert not deferred or seen[-1]                 # (the last call is the folded one)
+
+
+@pytest.mark.parametrize("arena", ["arena", "channels last"])
+def test_autoencoder_encoder(arena):
+    m = randomised(Encoder(VaeConfig(base=32, mult=(1, 2), layers_per_block=1), KW), seed=3)
+    no_further_than_plain_bf16(m, on_input([nhwc(1, 3, 32, 24)], lambda m, x: m(x)), arena)
